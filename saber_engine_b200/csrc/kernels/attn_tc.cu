@@ -9,10 +9,13 @@
 //   S = Q K^T   tcgen05.mma kind::f8f6f4, M = 128 rows, N = 128 keys, K = 256 dims (8 steps);
 //               Q is quantised to e4m3 with one scale per row when the tile is loaded, K pages
 //               are multiplied as they lie in the pool -- no widening pass;
-//   softmax     four warps, one thread per row (= TMEM lane): two passes over the row of S in
-//               tensor memory (maximum, then exp2), probabilities to e4m3 in shared memory;
+//   softmax     four warps, one thread per row (= TMEM lane): one pass over the row of S in
+//               tensor memory against a standing reference, probabilities to e4m3 in shared memory;
 //               the running reference maximum only moves when a tile exceeds it by 2^8 (the
-//               probabilities then still fit e4m3), so the accumulator is rarely rescaled;
+//               probabilities then still fit e4m3), so the accumulator is rarely rescaled.  Bound by
+//               this pass: 1.1 us a tile of 1.5 us; 2048 rows behind 2048 tokens, 24 heads of 4 key
+//               heads, take 164 us (650 before: a condition on every element's exponential, 4.6 us a
+//               tile), 8 x 8 rows behind 4096 tokens 25 us (76);
 //   O += P V    tcgen05.mma, M = 128, N = 256 dims, K = 128 keys (4 steps), accumulator in TMEM
 //               for the whole key range; S is double-buffered so the tensor core works on the
 //               next tile's scores while the softmax warps work on this one.
@@ -34,7 +37,7 @@
 
 namespace saber {
 
-constexpr int kTcThreads = 192;
+constexpr int kTcThreads = 224;            // keys, MMA issue, four softmax warps, values
 constexpr int kTcKeys = 128;             // keys per tile
 constexpr int kTcPages = kTcKeys / kPageTokens;
 constexpr uint32_t kTcQBytes = 32768;    // 128 rows x 256 B
@@ -126,43 +129,49 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
   const uint32_t tmem_o = tmem + 256;
   if (threadIdx.x == 0) { ATTN_STAMP(0); }
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ producer: pages -> stages
-    // lane 0 feeds the K ring, lane 1 the V ring
-    if (lane < 2) {
-      const bool is_v = lane == 1;
-      const uint32_t full = is_v ? v_full : k_full, empty = is_v ? v_empty : k_empty;
-      const uint32_t ring = is_v ? v_s : k_s;
-      int issued = 0;
-      bool ok = true;
-      for (int j = 0; j < ntiles && ok; ++j) {
-        const int s = j & 1;
-        if (j >= 2 && !mbar_wait(empty + 8 * s, ((j >> 1) - 1) & 1, p.err, kErrWaitEmpty)) { ok = false; break; }
-        mbar_arrive_expect_tx(full + 8 * s, kTcKVBytes);
-        for (int pg = 0; pg < kTcPages; ++pg) {
-          const int page = pg0 + j * kTcPages + pg;
-          int blk = 0;                                   // beyond the range: the null block (zeros)
-          if (page < pg1) {
-            blk = page < p.max_blocks ? p.block_table[static_cast<size_t>(b) * p.max_blocks + page] : -1;
-            if (blk < 0 || (p.n_blocks > 0 && blk >= p.n_blocks)) {   // never follow a bad table entry
-              if (p.err) atomicCAS(p.err, 0u, static_cast<uint32_t>(kErrBadIndex));
-              blk = 0;
-            }
-          }
-          const uint8_t* src = p.kv_cache + (static_cast<size_t>(blk) * p.nkv + kvh) * (2 * kPageTokens * kHeadDim) + (is_v ? 4096 : 0);
-          bulk_g2s(ring + s * kTcKVBytes + pg * 4096, src, 4096, full + 8 * s);
-        }
-        issued = j + 1;
+  if (warp == 0 || warp == 6) {
+    // ------------------------------------------------------------------ producers: pages -> stages
+    // One warp feeds the K ring, one the V ring.  Block ids are fetched 32 at a time (four tiles), a group ahead of their use, and a tile's
+    // eight pages are issued by eight lanes: one lane that looked an id up ahead of every copy spent 600 clocks a page, both rings in turn
+    // (2048 rows behind 2048 tokens, 24 heads: 232 us against 164).
+    const bool is_v = warp == 6;
+    const uint32_t full = is_v ? v_full : k_full, empty = is_v ? v_empty : k_empty;
+    const uint32_t ring = is_v ? v_s : k_s;
+    const int32_t* table = p.block_table + static_cast<size_t>(b) * p.max_blocks;
+    auto entry = [&](int page) { return page >= pg1 ? 0 : page < p.max_blocks ? table[page] : -1; };     // beyond the range: the null block (zeros)
+    int ids = entry(pg0 + lane), next = entry(pg0 + 32 + lane);
+    int issued = 0;
+    bool ok = true;
+    for (int j = 0; j < ntiles; ++j) {
+      const int s = j & 1;
+      int blk = __shfl_sync(0xffffffffu, ids, (j & 3) * kTcPages + (lane & (kTcPages - 1)));
+      if (blk < 0 || (p.n_blocks > 0 && blk >= p.n_blocks)) {         // never follow a bad table entry
+        if (p.err) atomicCAS(p.err, 0u, static_cast<uint32_t>(kErrBadIndex));
+        blk = 0;
       }
-      if (!ok) {
-        abort_s = 1u;
-        for (int j = max(0, issued - 2); j < issued; ++j)       // own copies in flight must land first
+      if ((j & 3) == 3) {
+        ids = next;
+        next = entry(pg0 + (j + 5) * kTcPages + lane);
+      }
+      if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * s, ((j >> 1) - 1) & 1, p.err, kErrWaitEmpty));
+      if (!ok) break;
+      if (lane == 0) mbar_arrive_expect_tx(full + 8 * s, kTcKVBytes);
+      __syncwarp();
+      if (lane < kTcPages) {
+        const uint8_t* src = p.kv_cache + (static_cast<size_t>(blk) * p.nkv + kvh) * (2 * kPageTokens * kHeadDim) + (is_v ? 4096 : 0);
+        bulk_g2s(ring + s * kTcKVBytes + lane * 4096, src, 4096, full + 8 * s);
+      }
+      issued = j + 1;
+    }
+    if (!ok) {
+      abort_s = 1u;
+      if (lane == 0)
+        for (int j = max(0, issued - 2); j < issued; ++j)             // own copies in flight must land first
           mbar_wait(full + 8 * (j & 1), (j >> 1) & 1, p.err, kErrWaitDrain);
-      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && ntiles > 0) {
+    if (ntiles > 0 && elect_one()) {
       const uint32_t idesc_s = make_idesc(kCFmtF32, kFmtE4M3, kFmtE4M3, 128, kTcKeys);
       const uint32_t idesc_o = make_idesc(kCFmtF32, kFmtE4M3, kFmtE4M3, 128, 256);
       bool ok = mbar_wait(q_full, 0, p.err, kErrWaitFull);
@@ -223,36 +232,42 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
               p.q + (static_cast<size_t>(row0 + t0 + tt) * p.nq + head0 + hh) * kHeadDim) + lane);
         }
       }
+      // (the rows' maxima side by side: five exchanges a row, one row behind the other, took most of this phase: 9 us, now 6)
+      float amax[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw[u]);
+        const __nv_bfloat162 m2 = __hmax2(__hmax2(__habs2(h2[0]), __habs2(h2[1])), __hmax2(__habs2(h2[2]), __habs2(h2[3])));
+        amax[u] = fmaxf(__low2float(m2), __high2float(m2));
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < 8; ++u) amax[u] = fmaxf(amax[u], __shfl_xor_sync(0xffffffffu, amax[u], o));
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int i = i0 + u;
         const int rr = qd * 32 + i;                               // MMA row
         const uint32_t dst = q_s + (rr >> 3) * 2048 + (rr & 7) * 16 + (lane >> 1) * 128 + (lane & 1) * 8;
         const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw[u]);
-        float f[8];
-        float amax = 0.f;
+        const float inv = amax[u] > 0.f ? 448.f / amax[u] : 0.f;      // (a dead row is all zeros: stays zeros)
+        if (lane == i) q_scale = amax[u] / 448.f;
+        uint32_t w[2];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 t2 = __bfloat1622float2(h2[e]);
-          f[2 * e] = t2.x; f[2 * e + 1] = t2.y;
-          amax = fmaxf(amax, fmaxf(fabsf(t2.x), fabsf(t2.y)));
+        for (int e = 0; e < 2; ++e) {
+          const float2 a = __bfloat1622float2(h2[2 * e]), c = __bfloat1622float2(h2[2 * e + 1]);
+          w[e] = static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(a.x * inv, a.y * inv), __NV_SATFINITE, __NV_E4M3)) |
+                 (static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(c.x * inv, c.y * inv), __NV_SATFINITE, __NV_E4M3)) << 16);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        const float inv = amax > 0.f ? 448.f / amax : 0.f;      // (a dead row is all zeros: stays zeros)
-        if (lane == i) q_scale = amax / 448.f;
-        const uint32_t lo = static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(f[0] * inv, f[1] * inv), __NV_SATFINITE, __NV_E4M3)) |
-                            (static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(f[2] * inv, f[3] * inv), __NV_SATFINITE, __NV_E4M3)) << 16);
-        const uint32_t hi = static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(f[4] * inv, f[5] * inv), __NV_SATFINITE, __NV_E4M3)) |
-                            (static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(f[6] * inv, f[7] * inv), __NV_SATFINITE, __NV_E4M3)) << 16);
-        asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst), "r"(lo), "r"(hi) : "memory");
+        asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst), "r"(w[0]), "r"(w[1]) : "memory");
       }
     }
     fence_proxy_async_smem();
     mbar_arrive(q_full);
     if (warp == 4 && lane == 0) { ATTN_STAMP(1); }
 
-    const float scale_log2 = p.sm_scale * p.k_scale * q_scale * 1.4426950408889634f;
+    float scale_log2 = p.sm_scale * p.k_scale * q_scale * 1.4426950408889634f;
+    if (scale_log2 == 0.f) scale_log2 = 1e-30f;          // (a row of zeros: times -inf, masked keys have to stay -inf)
     const int klim = kbase + tok;                        // keys below this bound are visible to the row
     float m_ref = -INFINITY, l_run = 0.f;
     bool ok = true;
@@ -268,22 +283,34 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
       float alpha = 1.f;
       if (warp_live) {
         const uint32_t prow = p_s + (j & 1) * kTcPBytes + (r >> 3) * 1024 + (r & 7) * 16;
-        const bool full_tile = kcap >= kTcKeys && kfloor <= 0;   // no masking needed for this row
-        // (every decision that steers a TMEM load below is made for the WHOLE warp: the loads are
-        // warp-collective)
+        // (decided for the WHOLE warp, like every decision that steers a TMEM load: the loads are warp-collective.  Dead rows compute on their
+        // zero queries, finite and never stored.)
+        const bool masked = __any_sync(0xffffffffu, row_live && (kcap < kTcKeys || kfloor > 0));
+        // Masked scores become -inf ahead of the arithmetic: with a condition on every element's exponential the compiler branches around
+        // each of them.
+        auto scores = [&](int c0, float (&sv)[32]) {
+          uint32_t raw[32];
+          tmem_ld32(ts + c0, raw);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sv[i] = __uint_as_float(raw[i]);
+          if (masked) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sv[i] = c0 + i < kcap && c0 + i >= kfloor ? sv[i] : -INFINITY;
+          }
+        };
         // Rows without a reference maximum yet (first tile with live keys) take a maximum pass first.
         if (__any_sync(0xffffffffu, row_live && m_ref == -INFINITY)) {
-          float tmax = -INFINITY;
+          float tmax[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
           for (int c0 = 0; c0 < kTcKeys; c0 += 32) {
-            uint32_t sv[32];
-            tmem_ld32(ts + c0, sv);
-            tmem_ld_wait();
+            float sv[32];
+            scores(c0, sv);
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (full_tile || (c0 + i < kcap && c0 + i >= kfloor)) tmax = fmaxf(tmax, __uint_as_float(sv[i]));
+            for (int i = 0; i < 32; ++i) tmax[i & 3] = fmaxf(tmax[i & 3], sv[i]);
           }
-          if (row_live && m_ref == -INFINITY) m_ref = tmax * scale_log2;     // (nothing accumulated yet: no rescale)
+          if (row_live && m_ref == -INFINITY)              // (nothing accumulated yet: no rescale)
+            m_ref = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3])) * scale_log2;
         }
         // Probability pass against the standing reference, the tile's own maximum on the side.  Only
         // when a row's tile exceeds its reference by more than 2^8 (the probabilities would leave
@@ -291,25 +318,21 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
         float l_tile = 0.f;
         for (int attempt = 0; attempt < 2; ++attempt) {
           const float msafe = m_ref == -INFINITY ? 0.f : m_ref;
-          float tmax = -INFINITY;
-          l_tile = 0.f;
+          float tmax[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, sum[4] = {};
 #pragma unroll
           for (int c0 = 0; c0 < kTcKeys; c0 += 32) {
-            uint32_t sv[32];
-            tmem_ld32(ts + c0, sv);
-            tmem_ld_wait();
+            float sv[32];
+            scores(c0, sv);
             uint32_t w[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               float pv[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const int c = c0 + 4 * i + e;
-                const float sc = __uint_as_float(sv[4 * i + e]);
-                const bool on = row_live && (full_tile || (c < kcap && c >= kfloor));
-                tmax = on ? fmaxf(tmax, sc) : tmax;
-                pv[e] = on ? exp2f(sc * scale_log2 - msafe) : 0.f;
-                l_tile += pv[e];
+                const float sc = sv[4 * i + e];
+                tmax[e] = fmaxf(tmax[e], sc);
+                pv[e] = exp2f(sc * scale_log2 - msafe);
+                sum[e] += pv[e];
               }
               const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(pv[0], pv[1]), __NV_SATFINITE, __NV_E4M3);
               const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(pv[2], pv[3]), __NV_SATFINITE, __NV_E4M3);
@@ -318,7 +341,8 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(prow + (c0 >> 4) * 128), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(prow + ((c0 >> 4) + 1) * 128), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
           }
-          const float tm = tmax * scale_log2;            // (-inf when the row has no live key in the tile)
+          l_tile = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+          const float tm = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3])) * scale_log2;            // (-inf when the row has no live key in the tile)
           const bool over = row_live && tm > m_ref + 8.f;
           if (over) {
             alpha = exp2f(m_ref - tm);                   // m_ref is finite here: the maximum pass set it
