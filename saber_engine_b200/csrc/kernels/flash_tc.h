@@ -22,6 +22,7 @@ struct FlashParams {
   int out_k0;
   int nseq, H, G, DK, V, VP, n_blocks, max_blocks, max_rows;
   int chunk;                  // > 0: a row sees the keys of its own chunk of positions only
+  int full;                   // every row sees every key of its sequence (DK <= 256 and VP <= 128)
   int window;                 // > 0: a row sees the last `window` keys only, its own among them
   float out_scale;
   float scale, softcap;       // softcap > 0: scores cap tanh(scale s / cap)

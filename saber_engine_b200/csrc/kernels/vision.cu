@@ -6,13 +6,15 @@
 // Parity: the reference tower's op list and rounding points (crates/saber-kernels/hip/vision.hip:1-30):
 // every linear rounds to bf16 once and the activation / residual work on the rounded value;
 // LayerNorm, softmax and rotary arithmetic run in fp32; rotated q and k are rounded to bf16; the
-// attention products run on mma.sync (bf16 operands, fp32 accumulators).
+// attention products run on tcgen05 (bf16 operands, fp32 accumulators).
 #include "vision.h"
+#include "flash_tc.h"
 #include "launch.cuh"
 
 namespace saber {
 
 constexpr int kVisThreads = 128;
+constexpr int kPrepThreads = 192;
 constexpr int kVisMaxChunks = 5;     // 8-value chunks per thread: rows of up to 5120 values
 
 __device__ __forceinline__ float block_sum128(float v, float* red) {
@@ -107,209 +109,91 @@ __global__ void __launch_bounds__(kVisThreads) vis_pos_add_kernel(const VisPosAd
   }
 }
 
-// ------------------------------------------------------------------------------------ rotary
-// In place on the q and k parts of qkv: out[d] = x[d] cos - x[d+36] sin, out[d+36] = x[d+36] cos + x[d] sin
-// (fp32 arithmetic, one rounding to bf16).  One CTA per row.
-constexpr int kHd = 72, kHalf = 36;
-
-__global__ void __launch_bounds__(kVisThreads) vis_rope_kernel(const VisAttnParams p, int rows) {
-  pdl_wait();
-  const int m = blockIdx.x;
-  if (m >= rows) return;
-  __nv_bfloat16* base = const_cast<__nv_bfloat16*>(p.qkv) + static_cast<size_t>(m) * p.ldq;
-  const float* cs = p.cos_t + static_cast<size_t>(m) * kHalf;
-  const float* sn = p.sin_t + static_cast<size_t>(m) * kHalf;
-  const int pairs = 2 * p.heads * kHalf;              // q heads, then k heads
-  for (int i = threadIdx.x; i < pairs; i += kVisThreads) {
-    const int hd = i / kHalf, d = i - hd * kHalf;     // hd < heads: q head, else k head (k starts at width = heads * 72)
-    __nv_bfloat16* x = base + hd * kHd;
-    const float x1 = __bfloat162float(x[d]), x2 = __bfloat162float(x[d + kHalf]);
-    x[d] = __float2bfloat16(x1 * cs[d] - x2 * sn[d]);
-    x[d + kHalf] = __float2bfloat16(x2 * cs[d] + x1 * sn[d]);
-  }
-}
-
 // ------------------------------------------------------------------------------------ attention
-// Non-causal attention inside one image on rotated q / k.  A CTA of four warps owns 64 query rows of
-// one head (16 per warp, the m16n8k16 tile).  Keys and values stream through a double-buffered
-// shared-memory ring, 64 rows at a time, by 16-byte asynchronous copies (rows past the image are
-// zero filled); both stay row-major -- row strides of 176 and 144 bytes put the eight rows of an
-// 8 x 8 matrix load on eight different 16-byte bank groups -- and reach the MMA as ldmatrix
-// fragments (values through the transposing form).  S = Q K^T and O += P V run on mma.sync with
-// fp32 accumulators; the softmax is the running-maximum form in the base-2 domain.
-constexpr int kKT = 64, kKStride = 88, kVStride = 72;
+// Non-causal attention inside each image, two launches: this one and the prompt attention of flash_tc.cu with every key visible.
+// A CTA takes 64 rows of one image and one head: q and k turned (out[d] = x[d] cos - x[d+36] sin, out[d+36] = x[d+36] cos + x[d] sin,
+// fp32, one rounding to bf16), q as rows of kVisDK values, k and the transposed v as the page of 64 keys that attention multiplies
+// in place.  Bound by memory: 7 KB in and 7 KB out per row, 11 us at 4096 rows (14 us for the rotation in place before, which left keys and
+// values in rows); all of a thread's loads are requested together.  With the attention behind it 147 us at 4096 rows (316 before) and 19 at 308
+// (13: three key blocks one behind the other in 32 CTAs are a longer chain than the 80 CTAs of `mma.sync` had).
+constexpr int kHd = 72, kHalf = 36;
+constexpr int kVisDK = 80, kVisKeyTiles = 2, kVisVP = 96;          // the head in whole steps of the tensor cores; values up to 32 columns
 
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ void vis_ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void vis_ldsm_x4_t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void vis_ldsm_x2_t(uint32_t addr, uint32_t (&r)[2]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
-               : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
-}
-// 16-byte asynchronous copy; src_bytes = 0 writes zeros
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+__device__ __forceinline__ float4 bf4(const uint2 v) {
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+  return make_float4(a.x, a.y, b.x, b.y);
 }
 
-__global__ void __launch_bounds__(kVisThreads, 4) vis_attn_kernel(const VisAttnParams p) {
-  __shared__ __align__(16) __nv_bfloat16 k_s[2][kKT][kKStride];
-  __shared__ __align__(16) __nv_bfloat16 v_s[2][kKT][kVStride];
+__device__ __forceinline__ uint2 bf4(float a, float b, float c, float d) {
+  __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+  return make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+
+// The rotated halves of four values of each half of a head row.
+__device__ __forceinline__ void rope4(const uint2 x1, const uint2 x2, const float4 c, const float4 s, uint2& lo, uint2& hi) {
+  const float4 a = bf4(x1), b = bf4(x2);
+  lo = bf4(a.x * c.x - b.x * s.x, a.y * c.y - b.y * s.y, a.z * c.z - b.z * s.z, a.w * c.w - b.w * s.w);
+  hi = bf4(b.x * c.x + a.x * s.x, b.y * c.y + a.y * s.y, b.z * c.z + a.z * s.z, b.w * c.w + a.w * s.w);
+}
+
+__global__ void __launch_bounds__(kPrepThreads) vis_prep_kernel(const VisAttnParams p) {
+  constexpr int kPer = 64 * 9 / kPrepThreads;
+  static_assert(kPer * kPrepThreads == 64 * 9 && kHalf == 36, "nine four-value groups of a half row, nine pieces of a row");
+  __shared__ __align__(16) uint8_t v_s[64 * kHd * 2 + 8 * 16];
   pdl_wait();
   const int4 blk = p.blocks[blockIdx.x];
-  const int seq0 = blk.x, len = blk.y, q0 = blk.z;
-  const int h = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  // the padding columns (head dim 72 -> 80) of the key tiles are never written again
-  for (int i = threadIdx.x; i < 2 * kKT * 8; i += kVisThreads)
-    k_s[i >> 9][(i >> 3) & (kKT - 1)][kHd + (i & 7)] = __float2bfloat16(0.f);
-  const __nv_bfloat16* kbase = p.qkv + static_cast<size_t>(seq0) * p.ldq + p.width + h * kHd;
-  auto issue = [&](int tile, int buf) {
-    const int k0 = tile * kKT;
-    for (int i = threadIdx.x; i < kKT * 9; i += kVisThreads) {
-      const int j = i / 9, c = i - j * 9;               // key row of the tile, 8-value chunk of the head
-      const bool in = k0 + j < len;
-      const __nv_bfloat16* kp = kbase + static_cast<size_t>(in ? k0 + j : 0) * p.ldq + c * 8;
-      cp_async16(static_cast<uint32_t>(__cvta_generic_to_shared(&k_s[buf][j][c * 8])), kp, in ? 16 : 0);
-      cp_async16(static_cast<uint32_t>(__cvta_generic_to_shared(&v_s[buf][j][c * 8])), kp + p.width, in ? 16 : 0);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  issue(0, 0);
-  // this warp's query fragments, straight from global memory (rows past the image read row 0, never stored)
-  uint32_t qf[5][4];
-  {
-    const int r0 = q0 + warp * 16 + g, r1 = r0 + 8;
-    const __nv_bfloat16* qa = p.qkv + static_cast<size_t>(seq0 + (r0 < len ? r0 : 0)) * p.ldq + h * kHd;
-    const __nv_bfloat16* qb = p.qkv + static_cast<size_t>(seq0 + (r1 < len ? r1 : 0)) * p.ldq + h * kHd;
+  const int h = blockIdx.y, m0 = blk.x + blk.z, n = min(64, blk.y - blk.z);
+  uint8_t* kp = p.k + (static_cast<size_t>(blockIdx.x) * p.heads + h) * kVisKeyTiles * 8192;
+  uint8_t* vp = p.v + (static_cast<size_t>(blockIdx.x) * p.heads + h) * kVisVP * 128;
+  uint2 q1[kPer], q2[kPer], k1[kPer], k2[kPer];
+  uint4 v[kPer];
+  float4 cs[kPer], sn[kPer];
 #pragma unroll
-    for (int ks = 0; ks < 5; ++ks) {
-      const int c0 = ks * 16 + 2 * t, c1 = c0 + 8;
-      qf[ks][0] = *reinterpret_cast<const uint32_t*>(qa + c0);
-      qf[ks][1] = *reinterpret_cast<const uint32_t*>(qb + c0);
-      qf[ks][2] = c1 < kHd ? *reinterpret_cast<const uint32_t*>(qa + c1) : 0u;
-      qf[ks][3] = c1 < kHd ? *reinterpret_cast<const uint32_t*>(qb + c1) : 0u;
+  for (int i = 0; i < kPer; ++i) {
+    const int e = threadIdx.x + i * kPrepThreads, r = e / 9, g = e - r * 9;
+    q1[i] = q2[i] = k1[i] = k2[i] = make_uint2(0u, 0u);            // (keys past the image: zeros, their probabilities are)
+    v[i] = make_uint4(0u, 0u, 0u, 0u);
+    cs[i] = sn[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < n) {
+      const __nv_bfloat16* row = p.qkv + static_cast<size_t>(m0 + r) * p.ldq + h * kHd;
+      q1[i] = *reinterpret_cast<const uint2*>(row + g * 4);
+      q2[i] = *reinterpret_cast<const uint2*>(row + kHalf + g * 4);
+      k1[i] = *reinterpret_cast<const uint2*>(row + p.width + g * 4);
+      k2[i] = *reinterpret_cast<const uint2*>(row + p.width + kHalf + g * 4);
+      v[i] = *reinterpret_cast<const uint4*>(row + 2 * p.width + g * 8);
+      cs[i] = *reinterpret_cast<const float4*>(p.cos_t + static_cast<size_t>(m0 + r) * kHalf + g * 4);
+      sn[i] = *reinterpret_cast<const float4*>(p.sin_t + static_cast<size_t>(m0 + r) * kHalf + g * 4);
     }
   }
-  const float qs = p.scale * 1.4426950408889634f;
-  float o[9][4];
 #pragma unroll
-  for (int j = 0; j < 9; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-  const int ntiles = (len + kKT - 1) / kKT;
-  // ldmatrix lane addressing: keys (lane & 7) + 8 * (lane >> 4) and column half (lane >> 3) & 1 for
-  // the key operand; keys (lane & 7) + 8 * ((lane >> 3) & 1) and dim block (lane >> 4) for values
-  const int kr = (lane & 7) + (lane >> 4) * 8, kc = ((lane >> 3) & 1) * 8;
-  const int vr = (lane & 7) + ((lane >> 3) & 1) * 8, vc = (lane >> 4) * 8;
-  for (int it = 0; it < ntiles; ++it) {
-    const int buf = it & 1;
-    if (it + 1 < ntiles) {
-      issue(it + 1, buf ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+  for (int i = 0; i < kPer; ++i) {
+    const int e = threadIdx.x + i * kPrepThreads, r = e / 9, g = e - r * 9;
+    *reinterpret_cast<uint4*>(v_s + r * (kHd * 2) + (r >> 3) * 16 + g * 16) = v[i];
+    auto key = [&](int col) { return kp + (col >> 6) * 8192 + r * 128 + ((((col >> 3) & 7) ^ (r & 7)) << 4) + (col & 7) * 2; };
+    uint2 lo, hi;
+    rope4(k1[i], k2[i], cs[i], sn[i], lo, hi);
+    *reinterpret_cast<uint2*>(key(g * 4)) = lo;
+    *reinterpret_cast<uint2*>(key(kHalf + g * 4)) = hi;
+    if (g == 8) *reinterpret_cast<uint4*>(key(kHd)) = make_uint4(0u, 0u, 0u, 0u);
+    if (r < n) {
+      __nv_bfloat16* q = p.q + (static_cast<size_t>(m0 + r) * p.heads + h) * kVisDK;
+      rope4(q1[i], q2[i], cs[i], sn[i], lo, hi);
+      *reinterpret_cast<uint2*>(q + g * 4) = lo;
+      *reinterpret_cast<uint2*>(q + kHalf + g * 4) = hi;
+      if (g == 8) *reinterpret_cast<uint4*>(q + kHd) = make_uint4(0u, 0u, 0u, 0u);
     }
-    __syncthreads();
-    const int valid = min(kKT, len - it * kKT);
-    const uint32_t kb = static_cast<uint32_t>(__cvta_generic_to_shared(&k_s[buf][0][0]));
-    const uint32_t vb = static_cast<uint32_t>(__cvta_generic_to_shared(&v_s[buf][0][0]));
-    float s[8][4];
-#pragma unroll
-    for (int np = 0; np < 4; ++np) {                    // pairs of 8-key score tiles
-      s[2 * np][0] = s[2 * np][1] = s[2 * np][2] = s[2 * np][3] = 0.f;
-      s[2 * np + 1][0] = s[2 * np + 1][1] = s[2 * np + 1][2] = s[2 * np + 1][3] = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < 5; ++ks) {
-        uint32_t b[4];
-        vis_ldsm_x4(kb + static_cast<uint32_t>(((np * 16 + kr) * kKStride + ks * 16 + kc) * 2), b);
-        mma_bf16(s[2 * np], qf[ks], b[0], b[1]);
-        mma_bf16(s[2 * np + 1], qf[ks], b[2], b[3]);
-      }
-    }
-    float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int key = nt * 8 + 2 * t + (c & 1);
-        s[nt][c] = key < valid ? s[nt][c] * qs : -INFINITY;
-      }
-      mx0 = fmaxf(mx0, fmaxf(s[nt][0], s[nt][1]));
-      mx1 = fmaxf(mx1, fmaxf(s[nt][2], s[nt][3]));
-    }
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-    const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);      // finite: key 0 of the tile is valid
-    const float c0 = exp2f(m0 - n0), c1 = exp2f(m1 - n1);      // 0 on the first tile
-    m0 = n0; m1 = n1;
-    l0 *= c0; l1 *= c1;
-#pragma unroll
-    for (int j = 0; j < 9; ++j) { o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1; }
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      s[nt][0] = exp2f(s[nt][0] - n0); s[nt][1] = exp2f(s[nt][1] - n0);
-      s[nt][2] = exp2f(s[nt][2] - n1); s[nt][3] = exp2f(s[nt][3] - n1);
-      l0 += s[nt][0] + s[nt][1];
-      l1 += s[nt][2] + s[nt][3];
-    }
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {                    // 16 keys per step: score tiles 2kk and 2kk + 1
-      uint32_t a[4];
-      a[0] = pack_bf16(s[2 * kk][0], s[2 * kk][1]);
-      a[1] = pack_bf16(s[2 * kk][2], s[2 * kk][3]);
-      a[2] = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]);
-      a[3] = pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
-      const uint32_t vrow = vb + static_cast<uint32_t>(((kk * 16 + vr) * kVStride + vc) * 2);
-#pragma unroll
-      for (int jp = 0; jp < 4; ++jp) {                  // dim blocks 2jp and 2jp + 1
-        uint32_t b[4];
-        vis_ldsm_x4_t(vrow + jp * 32, b);
-        mma_bf16(o[2 * jp], a, b[0], b[1]);
-        mma_bf16(o[2 * jp + 1], a, b[2], b[3]);
-      }
-      uint32_t b2[2];                                   // dim block 8 (lanes 16-31 repeat the addresses of 0-15)
-      vis_ldsm_x2_t(vb + static_cast<uint32_t>(((kk * 16 + vr) * kVStride + 64) * 2), b2);
-      mma_bf16(o[8], a, b2[0], b2[1]);
-    }
-    __syncthreads();                                    // this buffer is refilled by the next iteration's copies
   }
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-  const float i0 = 1.f / l0, i1 = 1.f / l1;
-  const int r0 = q0 + warp * 16 + g, r1 = r0 + 8;
+  __syncthreads();
+  for (int e = threadIdx.x; e < 8 * kHd / 2; e += kPrepThreads) {  // eight keys of two value columns (columns past the head are never read)
+    const int d = (e >> 3) * 2, c = e & 7;                         // the rows' pad of 16 bytes per eight puts the 32 lanes' words on 32 banks
+    uint32_t w[8];
 #pragma unroll
-  for (int j = 0; j < 9; ++j) {
-    const int ch = h * 9 + j;                           // 16-byte chunk of the output row (72 = 9 chunks per head)
-    const int kbk = ch >> 3, chunk = ch & 7;
-    if (r0 < len) {
-      const int mrow = seq0 + r0;
-      *reinterpret_cast<uint32_t*>(p.out_tiled + (static_cast<size_t>(kbk) * p.M_pad + mrow) * 128 +
-                                   ((chunk ^ (mrow & 7)) << 4) + 4 * t) = pack_bf16(o[j][0] * i0, o[j][1] * i0);
-    }
-    if (r1 < len) {
-      const int mrow = seq0 + r1;
-      *reinterpret_cast<uint32_t*>(p.out_tiled + (static_cast<size_t>(kbk) * p.M_pad + mrow) * 128 +
-                                   ((chunk ^ (mrow & 7)) << 4) + 4 * t) = pack_bf16(o[j][2] * i1, o[j][3] * i1);
-    }
+    for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const uint32_t*>(v_s + (c * 8 + j) * (kHd * 2) + c * 16 + d * 2);
+    uint4 o;
+    o.x = __byte_perm(w[0], w[1], 0x5410); o.y = __byte_perm(w[2], w[3], 0x5410); o.z = __byte_perm(w[4], w[5], 0x5410); o.w = __byte_perm(w[6], w[7], 0x5410);
+    *reinterpret_cast<uint4*>(vp + d * 128 + ((c ^ (d & 7)) << 4)) = o;
+    o.x = __byte_perm(w[0], w[1], 0x7632); o.y = __byte_perm(w[2], w[3], 0x7632); o.z = __byte_perm(w[4], w[5], 0x7632); o.w = __byte_perm(w[6], w[7], 0x7632);
+    *reinterpret_cast<uint4*>(vp + (d + 1) * 128 + ((c ^ ((d + 1) & 7)) << 4)) = o;
   }
 }
 
@@ -334,13 +218,39 @@ extern "C" int saber_vis_pos_add_launch(const saber::VisPosAddParams* p, cudaStr
 extern "C" int saber_vis_attn_launch(const saber::VisAttnParams* p, int n_blocks, cudaStream_t stream) {
   using namespace saber;
   if (n_blocks <= 0) return 0;
-  if ((p->width & 7) || p->heads * kHd != p->width || (p->ldq & 7)) return static_cast<int>(cudaErrorInvalidValue);
-  return static_cast<int>(saber::launch(vis_attn_kernel, dim3(n_blocks, p->heads), dim3(kVisThreads), 0, stream, 0, *p));
+  if ((p->width & 7) || p->heads * kHd != p->width || (p->ldq & 7) || p->images <= 0 || p->max_rows <= 0) return static_cast<int>(cudaErrorInvalidValue);
+  const cudaError_t e = launch(vis_prep_kernel, dim3(n_blocks, p->heads), dim3(kPrepThreads), 0, stream, 0, *p);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  FlashParams f = {};
+  f.q = p->q;
+  f.k = p->k;
+  f.v = p->v;
+  f.k_stride = static_cast<size_t>(kVisKeyTiles) * 8192;
+  f.v_stride = static_cast<size_t>(kVisVP) * 128;
+  f.cu_rows = p->cu_rows;
+  f.kv_len = p->kv_len;
+  f.block_table = p->pages;
+  f.out.p = p->out_tiled;
+  f.out.M_pad = p->M_pad;
+  f.nseq = p->images;
+  f.H = f.G = p->heads;
+  f.DK = kVisDK;
+  f.V = kHd;
+  f.VP = kVisVP;
+  f.n_blocks = n_blocks;
+  f.max_blocks = p->max_pages;
+  f.max_rows = p->max_rows;
+  f.full = 1;
+  f.out_scale = 1.f;
+  f.scale = p->scale;
+  f.err = p->err;
+  return saber_flash_tc(&f, stream);
 }
 
-extern "C" int saber_vis_rope_launch(const saber::VisAttnParams* p, int rows, cudaStream_t stream) {
+extern "C" int saber_vis_attn_scratch(int n_blocks, int rows, int heads, size_t* q, size_t* k, size_t* v) {
   using namespace saber;
-  if (rows <= 0) return 0;
-  if (p->heads * kHd != p->width) return static_cast<int>(cudaErrorInvalidValue);
-  return static_cast<int>(saber::launch(vis_rope_kernel, dim3(rows), dim3(kVisThreads), 0, stream, 0, *p, rows));
+  *q = static_cast<size_t>(rows) * heads * kVisDK * 2;
+  *k = static_cast<size_t>(n_blocks) * heads * kVisKeyTiles * 8192;
+  *v = static_cast<size_t>(n_blocks) * heads * kVisVP * 128;
+  return 0;
 }

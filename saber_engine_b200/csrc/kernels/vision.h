@@ -33,15 +33,20 @@ struct VisPosAddParams {
   int M, K;
 };
 
-// Non-causal attention inside each image; head dim 72.  The rotary kernel (in place on the q and k
-// parts of qkv, before the attention kernel) takes the same block; `blocks` rows cover 64 queries.
+// Non-causal attention inside each image; head dim 72.  q, k and v: scratch of the sizes that saber_vis_attn_scratch gives.
 struct VisAttnParams {
   const __nv_bfloat16* qkv; int ldq;     // [L][3 * width]: q | k | v, head-major inside each
   const float* cos_t; const float* sin_t; // [L][36]
   uint8_t* out_tiled; int M_pad;          // the projection GEMM's token operand (width columns)
-  const int4* blocks;                     // per CTA row block {first row of the image, rows of the image, first query (relative), 0}
+  const int4* blocks;                     // 64 rows of an image each {first row of the image, rows of the image, first row (relative), 0}
   int heads, width;
   float scale;                            // 1 / sqrt(72)
+  __nv_bfloat16* q; uint8_t* k; uint8_t* v;
+  const int32_t* cu_rows;                 // [images + 1]
+  const int32_t* kv_len;                  // [images]: rows of an image
+  const int32_t* pages;                   // [images][max_pages]: the blocks of an image
+  int images, max_pages, max_rows;
+  uint32_t* err;
 };
 
 }  // namespace saber
@@ -49,4 +54,4 @@ struct VisAttnParams {
 extern "C" int saber_vis_rows_launch(const saber::VisRowsParams* p, cudaStream_t stream);
 extern "C" int saber_vis_pos_add_launch(const saber::VisPosAddParams* p, cudaStream_t stream);
 extern "C" int saber_vis_attn_launch(const saber::VisAttnParams* p, int n_blocks, cudaStream_t stream);
-extern "C" int saber_vis_rope_launch(const saber::VisAttnParams* p, int rows, cudaStream_t stream);
+extern "C" int saber_vis_attn_scratch(int n_blocks, int rows, int heads, size_t* q, size_t* k, size_t* v);

@@ -163,7 +163,8 @@ class VisPosAddParams(C.Structure):
 
 class VisAttnParams(C.Structure):
     _fields_ = [("qkv", P), ("ldq", I), ("cos_t", P), ("sin_t", P), ("out_tiled", P), ("M_pad", I),
-                ("blocks", P), ("heads", I), ("width", I), ("scale", F)]
+                ("blocks", P), ("heads", I), ("width", I), ("scale", F), ("q", P), ("k", P), ("v", P), ("cu_rows", P), ("kv_len", P),
+                ("pages", P), ("images", I), ("max_pages", I), ("max_rows", I), ("err", P)]
 
 
 class Operand(C.Structure):
@@ -366,7 +367,7 @@ def _declare(L: C.CDLL) -> None:
         "saber_vis_rows_launch": (I, [C.POINTER(VisRowsParams), S]),
         "saber_vis_pos_add_launch": (I, [C.POINTER(VisPosAddParams), S]),
         "saber_vis_attn_launch": (I, [C.POINTER(VisAttnParams), I, S]),
-        "saber_vis_rope_launch": (I, [C.POINTER(VisAttnParams), I, S]),
+        "saber_vis_attn_scratch": (I, [I, I, I, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
         "saber_linear_launches": (I, [C.POINTER(LinParams)]),
         "saber_linear_launch": (I, [C.POINTER(LinParams), S]),
         "saber_stream_embed_launch": (I, [C.POINTER(StreamEmbedParams), S]),

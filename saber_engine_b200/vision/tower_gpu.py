@@ -1,7 +1,7 @@
 """The vision tower on the device: every linear is one launch of the tcgen05 GEMM in its bf16 mode
 (bias, GELU and the residual add in the epilogue), every normalisation writes the next GEMM's token
-operand directly, attention writes the projection's operand.  Attention is a rotary kernel in place on q / k and a
-flash-style mma.sync kernel.  Nine launches per block.
+operand directly, attention writes the projection's operand.  Attention is a kernel that turns q and k and lays keys and values out
+as pages, and the tcgen05 attention of prompt portions.  Nine launches per block.
 
     tower = VisionTowerGPU(cfg, weights, "cuda")
     rows = tower.forward(pixel_values, grids)        # bf16 [L / 4, out_hidden]
@@ -58,7 +58,7 @@ class VisionTowerGPU:
         self.m_ln = (m["ln_w"].float().to(d), m["ln_b"].float().to(d))
         self.m_fc1, self.m_fc2 = _Lin(m["fc1_w"], m["fc1_b"], d), _Lin(m["fc2_w"], m["fc2_b"], d)
         self.max_patches = max_patches
-        self._cap = 0
+        self._cap = self._blocks_cap = self._rows_cap = 0
         self.launches = 0
 
     # ------------------------------------------------------------------ buffers sized for L rows
@@ -74,7 +74,18 @@ class VisionTowerGPU:
         self.qkv = torch.empty(Lr, 3 * cfg.width, dtype=torch.bfloat16, device=d)
         self.h = torch.empty(Lr, L.round_up(cfg.mlp, 8), dtype=torch.bfloat16, device=d)
         self.mh = torch.empty((Lr + 3) // 4, cfg.width * cfg.merge ** 2, dtype=torch.bfloat16, device=d)
+        self._attn_scratch((Lr + 63) // 64 + 16, Lr)
         self._cap, self._m_pad_cap = Lr, m_pad
+
+    def _attn_scratch(self, blocks: int, rows: int) -> list:
+        """Turned queries, keys and values of one block's attention.  (Many small images have more blocks than `_reserve` foresaw: the
+        tables of a captured graph keep the buffers it was captured with.)"""
+        if blocks > self._blocks_cap or rows > self._rows_cap:
+            n = [C.c_size_t() for _ in range(3)]
+            N.lib().saber_vis_attn_scratch(blocks, rows, self.cfg.heads, *(C.byref(x) for x in n))
+            self._qkv = [torch.empty(x.value, dtype=torch.uint8, device=self.dev) for x in n]
+            self._blocks_cap, self._rows_cap = blocks, rows
+        return self._qkv
 
     # ------------------------------------------------------------------ launches
     def _rows(self, src: torch.Tensor, M: int, K: int, K_pad: int, m_pad: int, ln=None, group: int = 1) -> None:
@@ -107,7 +118,14 @@ class VisionTowerGPU:
         idx, wt = pos_gather_table(grids, cfg)
         cos, sin = rope_tables(grids, cfg)
         blocks = attn_blocks(grids)
-        return dict(idx=torch.from_numpy(idx).to(d), wt=torch.from_numpy(wt).to(d), cos=torch.from_numpy(cos).to(d),
+        rows = np.asarray([t * h * w for t, h, w in grids], dtype=np.int32)
+        per = (rows + 63) // 64
+        pages = np.zeros((len(grids), int(per.max())), dtype=np.int32)
+        for i, first in enumerate(np.concatenate([[0], np.cumsum(per)[:-1]])):
+            pages[i, :per[i]] = first + np.arange(per[i])
+        i32 = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).to(d)     # noqa: E731
+        return dict(cu_rows=i32(np.concatenate([[0], np.cumsum(rows)])), kv_len=i32(rows), pages=i32(pages), max_pages=pages.shape[1], max_rows=int(rows.max()),
+                    idx=torch.from_numpy(idx).to(d), wt=torch.from_numpy(wt).to(d), cos=torch.from_numpy(cos).to(d),
                     sin=torch.from_numpy(sin).to(d), blk=torch.from_numpy(blocks).to(d), n_blocks=int(blocks.shape[0]))
 
     def _run(self, px: torch.Tensor, Lr: int, meta: dict, out: Optional[torch.Tensor], stop_at_hidden: bool) -> None:
@@ -129,10 +147,13 @@ class VisionTowerGPU:
         pa.cos_t, pa.sin_t = meta["cos"].data_ptr(), meta["sin"].data_ptr()
         pa.out_tiled, pa.M_pad, pa.blocks = self.a_buf.data_ptr(), m_pad, meta["blk"].data_ptr()
         pa.heads, pa.width, pa.scale = cfg.heads, W, 1.0 / math.sqrt(cfg.head_dim)
+        meta["scratch"] = meta.get("scratch") or self._attn_scratch(meta["n_blocks"], Lr)
+        pa.q, pa.k, pa.v = (t.data_ptr() for t in meta["scratch"])
+        pa.cu_rows, pa.kv_len, pa.pages = (meta[k].data_ptr() for k in ("cu_rows", "kv_len", "pages"))
+        pa.images, pa.max_pages, pa.max_rows, pa.err = meta["kv_len"].numel(), meta["max_pages"], meta["max_rows"], F.scratch(self.dev).err.data_ptr()
         for b in self.blocks:
             self._rows(x, Lr, W, W, m_pad, ln=b["ln1"])
             self._gemm(b["qkv"], Lr, m_pad, qkv)
-            N.check(lib.saber_vis_rope_launch(C.byref(pa), Lr, N.stream_handle()), "vis_rope")
             N.check(lib.saber_vis_attn_launch(C.byref(pa), meta["n_blocks"], N.stream_handle()), "vis_attn")
             self.launches += 2
             self._gemm(b["proj"], Lr, m_pad, x, EPI_RES, res=x)
