@@ -49,8 +49,22 @@ struct VisAttnParams {
   uint32_t* err;
 };
 
+// out = epi(bf16(x W^T + bias)): epi 1 gelu (by tanh), 2 gelu (by the error function), 3 + res; bf16 rows (vis_linear.cu).
+struct VisLinearParams {
+  const uint8_t* w;        // [N_pad / 256][k-block of 64][256 rows of 128 bytes]
+  const uint8_t* a;        // [k-block][M_pad][128 bytes]
+  const float* bias;       // [N] or null
+  const __nv_bfloat16* res; // epi 3: out's row stride, may alias out
+  __nv_bfloat16* out;      // [M][ldo]
+  float* ws;               // an SM: 128 x 256 floats
+  uint32_t* counters;      // an SM: a word, zero between launches
+  uint32_t* err;
+  int M, M_pad, N, N_pad, K, ldo, epi;
+};
+
 }  // namespace saber
 
+extern "C" int saber_vis_linear_launch(const saber::VisLinearParams* p, cudaStream_t stream);
 extern "C" int saber_vis_rows_launch(const saber::VisRowsParams* p, cudaStream_t stream);
 extern "C" int saber_vis_pos_add_launch(const saber::VisPosAddParams* p, cudaStream_t stream);
 extern "C" int saber_vis_attn_launch(const saber::VisAttnParams* p, int n_blocks, cudaStream_t stream);

@@ -167,6 +167,11 @@ class VisAttnParams(C.Structure):
                 ("pages", P), ("images", I), ("max_pages", I), ("max_rows", I), ("err", P)]
 
 
+class VisLinearParams(C.Structure):
+    _fields_ = [("w", P), ("a", P), ("bias", P), ("res", P), ("out", P), ("ws", P), ("counters", P), ("err", P),
+                ("M", I), ("M_pad", I), ("N", I), ("N_pad", I), ("K", I), ("ldo", I), ("epi", I)]
+
+
 class Operand(C.Structure):
     """Token operand of a linear: bf16 GEMM tiles (fmt 0) or fp32 rows (fmt 1)."""
     _fields_ = [("p", P), ("M_pad", I), ("ld", I), ("fmt", I)]
@@ -367,6 +372,7 @@ def _declare(L: C.CDLL) -> None:
         "saber_vis_rows_launch": (I, [C.POINTER(VisRowsParams), S]),
         "saber_vis_pos_add_launch": (I, [C.POINTER(VisPosAddParams), S]),
         "saber_vis_attn_launch": (I, [C.POINTER(VisAttnParams), I, S]),
+        "saber_vis_linear_launch": (I, [C.POINTER(VisLinearParams), S]),
         "saber_vis_attn_scratch": (I, [I, I, I, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
         "saber_linear_launches": (I, [C.POINTER(LinParams)]),
         "saber_linear_launch": (I, [C.POINTER(LinParams), S]),

@@ -1,5 +1,5 @@
-"""The vision tower on the device: every linear is one launch of the tcgen05 GEMM in its bf16 mode
-(bias, GELU and the residual add in the epilogue), every normalisation writes the next GEMM's token
+"""The vision tower on the device: every linear is one launch of a bf16 tcgen05 product (`vis_linear.cu`;
+bias, GELU and the residual add in the epilogue), every normalisation writes the next GEMM's token
 operand directly, attention writes the projection's operand.  Attention is a kernel that turns q and k and lays keys and values out
 as pages, and the tcgen05 attention of prompt portions.  Nine launches per block.
 
@@ -75,6 +75,7 @@ class VisionTowerGPU:
         self.h = torch.empty(Lr, L.round_up(cfg.mlp, 8), dtype=torch.bfloat16, device=d)
         self.mh = torch.empty((Lr + 3) // 4, cfg.width * cfg.merge ** 2, dtype=torch.bfloat16, device=d)
         self._attn_scratch((Lr + 63) // 64 + 16, Lr)
+        self._workspace()
         self._cap, self._m_pad_cap = Lr, m_pad
 
     def _attn_scratch(self, blocks: int, rows: int) -> list:
@@ -86,6 +87,14 @@ class VisionTowerGPU:
             self._qkv = [torch.empty(x.value, dtype=torch.uint8, device=self.dev) for x in n]
             self._blocks_cap, self._rows_cap = blocks, rows
         return self._qkv
+
+    def _workspace(self) -> tuple:
+        """Partial sums of cut reductions: at most a 256-feature tile per SM, and a counter.  (The tower runs beside the step loop: a workspace
+        of its own.)"""
+        if getattr(self, "_parts", None) is None:
+            sms = F.device_sms()
+            self._parts = torch.empty(sms * 256 * 128, dtype=torch.float32, device=self.dev), torch.zeros(sms, dtype=torch.int32, device=self.dev)
+        return self._parts
 
     # ------------------------------------------------------------------ launches
     def _rows(self, src: torch.Tensor, M: int, K: int, K_pad: int, m_pad: int, ln=None, group: int = 1) -> None:
@@ -99,16 +108,13 @@ class VisionTowerGPU:
 
     def _gemm(self, lin: _Lin, M: int, m_pad: int, out: torch.Tensor, epi: int = EPI_NONE,
               res: Optional[torch.Tensor] = None, k_pad: Optional[int] = None) -> None:
-        sc = F.scratch(self.dev)
-        p = N.GemmI8Params()
-        p.w, p.w_scale, p.a, p.a_scale = lin.tiles.data_ptr(), None, self.a_buf.data_ptr(), None
-        p.out, p.ws, p.counters, p.err = out.data_ptr(), sc.ws.data_ptr(), sc.counters.data_ptr(), sc.err.data_ptr()
-        p.M, p.M_pad, p.N, p.N_pad, p.K = M, m_pad, lin.N, lin.N_pad, (k_pad or lin.K_pad) * 2
-        p.nt, p.splits, p.w4, p.ldo = L.token_tile(M), 1, 3, out.stride(0)
-        p.mtiles = getattr(self, "force_pairs", 0)     # tests set 2 to run the paired-tile path on small shapes
+        p = N.VisLinearParams()
+        p.w, p.a, p.out, p.err = lin.tiles.data_ptr(), self.a_buf.data_ptr(), out.data_ptr(), F.scratch(self.dev).err.data_ptr()
+        p.ws, p.counters = (t.data_ptr() for t in self._workspace())
+        p.M, p.M_pad, p.N, p.N_pad, p.K, p.ldo = M, m_pad, lin.N, lin.N_pad, k_pad or lin.K_pad, out.stride(0)
         p.bias, p.epi, p.res = lin.bias.data_ptr(), epi, (res.data_ptr() if res is not None else None)
         assert out.stride(0) % 8 == 0 and (res is None or res.stride(0) == out.stride(0))
-        N.check(N.lib().saber_gemm_i8_launch(C.byref(p), 0, N.stream_handle()), "vision gemm")
+        N.check(N.lib().saber_vis_linear_launch(C.byref(p), N.stream_handle()), "vision linear")
         self.launches += 1
 
     # ------------------------------------------------------------------ forward
