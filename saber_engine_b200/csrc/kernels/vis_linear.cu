@@ -98,6 +98,7 @@ __device__ __forceinline__ void vis_linear_store(const VisLinearParams& p, const
 
 // grid: resident CTAs; item i is part i / tiles of tile i % tiles
 __global__ void __launch_bounds__(kVlThreads, 1) vis_linear_kernel(const __grid_constant__ VisLinearParams p, const VisLinearShape sh) {
+  pdl_trigger();                                   // (one round of CTAs: the next kernel may get ready beside them; it waits before it reads or writes)
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bars[2 * kVlStages + 5];
   __shared__ uint32_t tmem_base_s, last_s;

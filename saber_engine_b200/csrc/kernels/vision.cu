@@ -17,9 +17,12 @@ constexpr int kVisThreads = 128;
 constexpr int kPrepThreads = 192;
 constexpr int kVisMaxChunks = 5;     // 8-value chunks per thread: rows of up to 5120 values
 
-__device__ __forceinline__ float block_sum128(float v, float* red) {
+// kLanes 32: a row per warp, four a CTA; 128: a row per CTA.
+template <int kLanes>
+__device__ __forceinline__ float row_sum(float v, float* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if constexpr (kLanes == 32) return v;
   const int w = threadIdx.x >> 5;
   __syncthreads();                       // red may still be read from the previous call
   if ((threadIdx.x & 31) == 0) red[w] = v;
@@ -27,20 +30,25 @@ __device__ __forceinline__ float block_sum128(float v, float* red) {
   return red[0] + red[1] + red[2] + red[3];
 }
 
+// Bound by memory (3 us for 4096 rows of 1152 at the copy rate).  A row per warp wherever it holds one: a row per CTA left most of the 128 threads
+// without a second chunk and met at four barriers, and a condition beside every element's norm weight was a branch an element
+// (15.4 us a launch; a 64 x 64 image has 84 of them and takes 9.1 ms, 9.7 before).
+template <int kLanes, bool kF32>
 __global__ void __launch_bounds__(kVisThreads) vis_rows_kernel(const VisRowsParams p) {
   __shared__ float red[4];
+  pdl_trigger();
   pdl_wait();
-  const int m = blockIdx.x;
-  const int nch = p.K_pad >> 3;
+  const int t = threadIdx.x & (kLanes - 1), m = blockIdx.x * (kVisThreads / kLanes) + threadIdx.x / kLanes;
+  if (m >= p.M) return;
+  const int nch = p.K_pad >> 3, live = p.K >> 3;
   float v[kVisMaxChunks][8];
-  float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < kVisMaxChunks; ++i) {
-    const int c = threadIdx.x + i * kVisThreads;
+    const int c = t + i * kLanes;
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[i][j] = 0.f;
-    if (c < nch && c * 8 < p.K) {
-      if (p.x_f32) {
+    if (c < live) {
+      if constexpr (kF32) {
         const float4* s = reinterpret_cast<const float4*>(static_cast<const float*>(p.x) + static_cast<size_t>(m) * p.ldx + c * 8);
         const float4 a = s[0], b = s[1];
         v[i][0] = a.x; v[i][1] = a.y; v[i][2] = a.z; v[i][3] = a.w;
@@ -51,39 +59,45 @@ __global__ void __launch_bounds__(kVisThreads) vis_rows_kernel(const VisRowsPara
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[i][j] = __bfloat162float(b[j]);
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) sum += v[i][j];
     }
   }
-  float mean = 0.f, rstd = 1.f;
   if (p.ln_w != nullptr) {
-    mean = block_sum128(sum, red) / static_cast<float>(p.K);
-    float sq = 0.f;
+    float sum = 0.f, sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < kVisMaxChunks; ++i) {
-      const int c = threadIdx.x + i * kVisThreads;
-      if (c < nch && c * 8 < p.K) {
+    for (int i = 0; i < kVisMaxChunks; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum += v[i][j];                    // (chunks past the row are zeros)
+    const float mean = row_sum<kLanes>(sum, red) / static_cast<float>(p.K);
+#pragma unroll
+    for (int i = 0; i < kVisMaxChunks; ++i)
+      if (t + i * kLanes < live) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) { const float d = v[i][j] - mean; sq += d * d; }
       }
+    const float rstd = rsqrtf(row_sum<kLanes>(sq, red) / static_cast<float>(p.K) + p.eps);
+#pragma unroll
+    for (int i = 0; i < kVisMaxChunks; ++i) {
+      const int c = t + i * kLanes;
+      if (c < live) {
+        const float4* w4 = reinterpret_cast<const float4*>(p.ln_w + c * 8);
+        const float4* b4 = reinterpret_cast<const float4*>(p.ln_b + c * 8);
+        const float4 w0 = w4[0], w1 = w4[1], b0 = b4[0], b1 = b4[1];
+        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w}, b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[i][j] = (v[i][j] - mean) * rstd * w[j] + b[j];
+      }
     }
-    rstd = rsqrtf(block_sum128(sq, red) / static_cast<float>(p.K) + p.eps);
   }
   const int row_o = m / p.group;
   const int col_base = (m % p.group) * p.K;
 #pragma unroll
   for (int i = 0; i < kVisMaxChunks; ++i) {
-    const int c = threadIdx.x + i * kVisThreads;
-    if (c >= nch) continue;
+    const int c = t + i * kLanes;
+    if (c >= nch) break;
     uint4 o;
     __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(&o);
-    const bool in = c * 8 < p.K;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float y = v[i][j];
-      if (in && p.ln_w != nullptr) y = (y - mean) * rstd * p.ln_w[c * 8 + j] + p.ln_b[c * 8 + j];
-      ob[j] = __float2bfloat16(in ? y : 0.f);
-    }
+    for (int j = 0; j < 8; ++j) ob[j] = __float2bfloat16(v[i][j]);   // (zeros up to the operand's end)
     const int col0 = col_base + c * 8;
     const int kb = col0 >> 6, chunk = (col0 & 63) >> 3;
     *reinterpret_cast<uint4*>(p.tiled + (static_cast<size_t>(kb) * p.M_pad + row_o) * 128 +
@@ -206,7 +220,10 @@ extern "C" int saber_vis_rows_launch(const saber::VisRowsParams* p, cudaStream_t
       (p->group != 1 && p->group != 4) || (p->group == 1 && (p->K_pad & 63)) ||
       (p->group > 1 && ((p->K & 63) || p->K_pad != p->K)) || (p->ldx & 7) || (p->M + p->group - 1) / p->group > p->M_pad)
     return static_cast<int>(cudaErrorInvalidValue);
-  return static_cast<int>(saber::launch(vis_rows_kernel, dim3(p->M), dim3(kVisThreads), 0, stream, 0, *p));
+  const dim3 warps((p->M + 3) / 4), ctas(p->M), threads(kVisThreads);
+  if (p->K_pad <= kVisMaxChunks * 32 * 8)
+    return static_cast<int>(p->x_f32 ? launch(vis_rows_kernel<32, true>, warps, threads, 0, stream, 0, *p) : launch(vis_rows_kernel<32, false>, warps, threads, 0, stream, 0, *p));
+  return static_cast<int>(p->x_f32 ? launch(vis_rows_kernel<128, true>, ctas, threads, 0, stream, 0, *p) : launch(vis_rows_kernel<128, false>, ctas, threads, 0, stream, 0, *p));
 }
 
 extern "C" int saber_vis_pos_add_launch(const saber::VisPosAddParams* p, cudaStream_t stream) {

@@ -48,14 +48,15 @@ class VisionTowerGPU:
         d = self.dev
         self.patch = _Lin(wts.patch_w, wts.patch_b, d)
         self.pos_table = wts.pos_table.to(torch.bfloat16).to(d).contiguous()
+        vec = lambda t: t.float().to(d).clone()         # noqa: E731  (storage of its own: read 16 bytes at a time)
         self.blocks = []
         for b in wts.blocks:
             self.blocks.append(dict(
-                ln1=(b["ln1_w"].float().to(d), b["ln1_b"].float().to(d)), qkv=_Lin(b["qkv_w"], b["qkv_b"], d),
-                proj=_Lin(b["proj_w"], b["proj_b"], d), ln2=(b["ln2_w"].float().to(d), b["ln2_b"].float().to(d)),
+                ln1=(vec(b["ln1_w"]), vec(b["ln1_b"])), qkv=_Lin(b["qkv_w"], b["qkv_b"], d),
+                proj=_Lin(b["proj_w"], b["proj_b"], d), ln2=(vec(b["ln2_w"]), vec(b["ln2_b"])),
                 fc1=_Lin(b["fc1_w"], b["fc1_b"], d), fc2=_Lin(b["fc2_w"], b["fc2_b"], d)))
         m = wts.merger
-        self.m_ln = (m["ln_w"].float().to(d), m["ln_b"].float().to(d))
+        self.m_ln = (vec(m["ln_w"]), vec(m["ln_b"]))
         self.m_fc1, self.m_fc2 = _Lin(m["fc1_w"], m["fc1_b"], d), _Lin(m["fc2_w"], m["fc2_b"], d)
         self.max_patches = max_patches
         self._cap = self._blocks_cap = self._rows_cap = 0
