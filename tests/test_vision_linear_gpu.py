@@ -1,4 +1,4 @@
-"""The tower's linears against float64 of the same bf16 operands."""
+"""The tower's rows and linears against float64 of the same operands."""
 import ctypes as C
 
 import pytest
@@ -51,3 +51,37 @@ def test_linear_matches_float64(M, N_, K, epi):
     bound = 1.2 * 2.0 ** -8 * y.abs() + 2.0 ** -8 * want.abs() * (1 + 2.0 ** -8) + K * 2.0 ** -24 * size + (2.0 ** -11 * y.abs() if epi in (1, 2) else 0)
     assert bool(((out[:, :N_].double() - want).abs() <= bound + 1e-6).all())
     assert bool((out[:, N_:] == 7.0).all())
+
+
+# A row per warp up to 1280 columns, per CTA beyond; ragged last warps; rows grouped by four; fp32 and bf16 rows.
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,K,group", [(1, 72, 1), (5, 1152, 1), (130, 1280, 1), (33, 1288, 1), (9, 4608, 1), (6, 128, 4), (40, 1152, 4), (8, 1344, 4)])
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rows_match_float64(M, K, group, norm, dtype):
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = (torch.randn(M, K, generator=g, device="cuda") * 3 + 1).to(dtype)
+    w, b = torch.randn(K, generator=g, device="cuda"), torch.randn(K, generator=g, device="cuda")
+    k_pad, rows = (K + 63) // 64 * 64, (M + group - 1) // group
+    m_pad = (rows + 31) // 32 * 32
+    out = torch.full((k_pad * group // 64, m_pad, 8, 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    p = N.VisRowsParams()
+    p.x, p.x_f32, p.ldx, p.tiled, p.eps = x.data_ptr(), int(dtype == torch.float32), K, out.data_ptr(), 1e-6
+    p.ln_w, p.ln_b = (w.data_ptr(), b.data_ptr()) if norm else (None, None)
+    p.M, p.K, p.K_pad, p.M_pad, p.group = M, K, k_pad, m_pad, group
+    N.check(N.lib().saber_vis_rows_launch(C.byref(p), N.stream_handle()), "vis_rows")
+    torch.cuda.synchronize()
+    at = torch.arange(8, device="cuda")[None, :] ^ (torch.arange(m_pad, device="cuda")[:, None] & 7)
+    got = torch.gather(out, 2, at[None, :, :, None].expand(out.shape[0], -1, -1, 8)).transpose(0, 1).reshape(m_pad, -1)[:rows].double()
+    want = x.double()
+    size = torch.zeros_like(want)
+    if norm:
+        d = want - want.mean(-1, keepdim=True)
+        f = torch.rsqrt((d * d).mean(-1, keepdim=True) + 1e-6)
+        want, size = d * f * w.double() + b.double(), (d * f * w.double()).abs() + b.double().abs()
+    full = torch.zeros(rows * group, K if group > 1 else k_pad, dtype=torch.float64, device="cuda")
+    room = torch.zeros_like(full)
+    full[:M, :K], room[:M, :K] = want, 2.0 ** -8 * want.abs() + 2.0 ** -16 * size              # one rounding to bf16; fp32 sums of a row
+    got, full, room = got[:, :full.shape[1] * group], full.view(rows, -1), room.view(rows, -1)
+    live = torch.arange(rows * group, device="cuda").view(rows, group).repeat_interleave(full.shape[1] // group, 1) < M
+    assert bool(((got - full).abs() <= room)[live].all())
