@@ -1,6 +1,7 @@
 // Gated delta rule with free head sizes, fp32 throughout.
 //
-// Prompt portions (ragged rows, any length), in blocks of four tokens: three launches.
+// Prompt portions (ragged rows, any length): three launches, the first two those of delta_chunk.cu where a chunk scratch is given (bf16 models), else,
+// in blocks of four tokens:
 //   prep   convolution, silu, unit norms, beta and decay, and per block the dot products k_j . k_i and k_j . q_i
 //   scan   the recurrence.  Columns of the state are independent, so a warp owns four value columns for the
 //          whole portion: sixteen lanes split the key dimension, two lane groups take two columns each, the state
@@ -622,8 +623,13 @@ static int delta_go(const DeltaParams& p, bool single, cudaStream_t stream) {
     const int smem = (2 * NI * 32 + 2 * p.VP) * 4;
     return static_cast<int>(launch(delta_step_kernel<NI>, dim3(p.H, p.nseq), dim3(32 * warps), smem, stream, 0, p));
   }
-  int e = static_cast<int>(p.taps == 4 ? delta_prep<NI, 4>(p, stream) : delta_prep<NI, 0>(p, stream));
-  if (e == 0) e = delta_scan<NJ, true>(p, stream);
+  int e;
+  if (p.chunk != nullptr) {
+    e = saber_delta_chunk_launch(&p, stream);
+  } else {
+    e = static_cast<int>(p.taps == 4 ? delta_prep<NI, 4>(p, stream) : delta_prep<NI, 0>(p, stream));
+    if (e == 0) e = delta_scan<NJ, true>(p, stream);
+  }
   if (e == 0) e = static_cast<int>(launch(delta_out_kernel, dim3(p.M + p.nseq, (p.H + 7) / 8), dim3(256), 0, stream, 0, p));
   return e;
 }

@@ -35,6 +35,7 @@ struct DeltaParams {
   float eps, unit_eps, q_scale;
   const float* skip;       // [H] or null: the scan without correction adds skip * v to the read-out
   uint32_t* err;
+  float* chunk;            // scratch of saber_delta_chunk_floats: prompt portions go sixteen tokens at a time on the tensor cores (bf16 models); null: the scan
 };
 
 }  // namespace saber
@@ -42,6 +43,9 @@ struct DeltaParams {
 // rows = 1: every sequence brings at most one row (one fused launch); else three launches
 extern "C" int saber_delta_launches(int single_row);
 extern "C" int saber_delta_launch(const saber::DeltaParams* p, int single_row, cudaStream_t stream);
+// Scratch of the chunk form in floats (0: it does not take these sizes), and its first two launches (delta_chunk.cu)
+extern "C" size_t saber_delta_chunk_floats(const saber::DeltaParams* p);
+int saber_delta_chunk_launch(const saber::DeltaParams* p, cudaStream_t stream);
 // The scan by itself over records that another kernel has prepared, with the rule S <- g S + beta k v^T (no
 // correction of v by what the state holds): decayed outer products (ssd.cu).
 int saber_outer_scan_launch(const saber::DeltaParams* p, cudaStream_t stream);

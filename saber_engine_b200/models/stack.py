@@ -467,7 +467,7 @@ class StackModel:
         mx = lambda it: max(it, default=0)    # noqa: E731
         wk = {"splits": self._splits(M, decode)}
         if not decode:
-            floats = {id(m): self._chunk_floats(m, M, nseq) for m in outer}
+            floats = {id(m): self._chunk_floats(m, M, nseq) for m in ms if isinstance(m, (DeltaMixer, OuterMixer))}
             scan = [m for m in de if not floats.get(id(m))]
             blk = M // 4 + nseq                           # blocks of four tokens
             wk["kq"] = f32(blk * mx(m.kv_heads * (8 * m.dim_pad + 16) for m in scan))
@@ -518,10 +518,14 @@ class StackModel:
         """Key splits of the absorbed attention: fill the SMs once."""
         return max(1, min(32, F.device_sms() // max(1, M))) if decode or M < 64 else 1
 
-    def _chunk_floats(self, m: OuterMixer, M: int, nseq: int) -> int:
-        """Scratch of the chunk form for prompt portions (0: the scan serves: fp32, or sizes it does not take)."""
+    def _chunk_floats(self, m, M: int, nseq: int) -> int:
+        """Scratch of a recurrent mixer's chunk form for prompt portions (0: the scan serves: fp32, or sizes it does not take)."""
         if self.f32:
             return 0
+        if isinstance(m, DeltaMixer):
+            p = N.DeltaParams()
+            p.M, p.nseq, p.H, p.HK, p.DP, p.VP = M, nseq, m.heads, m.kv_heads, m.dim_pad, m.vdim_pad
+            return N.lib().saber_delta_chunk_floats(C.byref(p))
         p = N.SsdParams()
         p.M, p.nseq, p.H, p.HK, p.N, p.DP, p.V, p.VP, p.taps = M, nseq, m.heads, m.kv_heads, m.dim, m.dim_pad, m.vdim, m.vdim_pad, m.taps
         return N.lib().saber_ssd_chunk_floats(C.byref(p))
@@ -611,6 +615,8 @@ class StackModel:
         p.conv_w, p.A_log, p.dt_bias, p.norm_w = (lw.extra[k].data_ptr() for k in ("conv", "A_log", "dt_bias", "norm"))
         p.hist, p.state = self.hist[run.index].data_ptr(), self.state[run.index].data_ptr()
         p.kq, p.vb, p.o = (N.ptr(wk.get(k)) for k in ("kq", "vb", "o"))
+        if "chunk" in wk and self._chunk_floats(m, M, nseq):
+            p.chunk = wk["chunk"].data_ptr()
         p.cu_rows, p.slots, p.pos = at(lay.cu_rows), at(lay.slots), at(lay.pos)
         p.out, p.out_k0, p.M, p.nseq = m_op, 0, M, nseq
         p.H, p.HK, p.D, p.DP, p.V, p.VP, p.taps, p.n_slots = m.heads, m.kv_heads, m.dim, m.dim_pad, m.vdim, m.vdim_pad, m.taps, self.n_slots

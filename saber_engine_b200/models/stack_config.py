@@ -689,11 +689,14 @@ class StackConfig:
         return max([rows * l.mlp.top * elem * (l.mlp.ff + self.width) for l in self.layers if isinstance(l.mlp, ExpertMix)], default=0)
 
     def scan_row_bytes(self, rows: int) -> int:
-        """Scratch of the prompt scans of channel delta rules and of convolved queries, keys and values (one layer at a time)."""
+        """Scratch of the prompt scans of delta rules and of convolved queries, keys and values (one layer at a time)."""
         n = [0]
         for m in self.mixers():
             if isinstance(m, ChannelDeltaMixer):
                 n.append(m.heads * (17 * m.dim_pad + 64 + 4 * m.vdim_pad + 128) // 4 + m.heads * m.vdim_pad)
+            elif isinstance(m, DeltaMixer):
+                slices = (m.vdim_pad + 31) // 32
+                n.append((m.kv_heads * 192 * m.dim_pad + m.heads * (2304 * slices + 4864)) // 64 + m.heads * m.vdim_pad)
             elif isinstance(m, GroupedMixer) and m.taps:
                 n.append(m.channels + 32)
         return 4 * rows * max(n)

@@ -204,7 +204,7 @@ class DeltaParams(C.Structure):
     _fields_ = [("x", P), ("ldx", I), ("q_off", I), ("k_off", I), ("v_off", I), ("b_off", I), ("a_off", I), ("g_off", I), ("conv_w", P),
                 ("A_log", P), ("dt_bias", P), ("norm_w", P), ("hist", P), ("state", P), ("kq", P), ("vb", P), ("o", P),
                 ("cu_rows", P), ("slots", P), ("pos", P), ("out", Operand), ("out_k0", I), ("M", I), ("nseq", I), ("H", I), ("HK", I),
-                ("D", I), ("DP", I), ("V", I), ("VP", I), ("taps", I), ("n_slots", I), ("eps", F), ("unit_eps", F), ("q_scale", F), ("skip", P), ("err", P)]
+                ("D", I), ("DP", I), ("V", I), ("VP", I), ("taps", I), ("n_slots", I), ("eps", F), ("unit_eps", F), ("q_scale", F), ("skip", P), ("err", P), ("chunk", P)]
 
 
 class MlaParams(C.Structure):
@@ -383,6 +383,7 @@ def _declare(L: C.CDLL) -> None:
         "saber_mla_launch": (I, [C.POINTER(MlaParams), S]),
         "saber_ssd_launch": (I, [C.POINTER(SsdParams), I, S]),
         "saber_ssd_chunk_floats": (C.c_size_t, [C.POINTER(SsdParams)]),
+        "saber_delta_chunk_floats": (C.c_size_t, [C.POINTER(DeltaParams)]),
         "saber_gqa_form": (I, [C.POINTER(GqaParams)]),
         "saber_gqa_launch": (I, [C.POINTER(GqaParams), S]),
         "saber_cdelta_launch": (I, [C.POINTER(CdeltaParams), I, S]),
