@@ -1,6 +1,7 @@
 // Delta rule with a decay and a removal rate per key channel, free head sizes, fp32 throughout.
 //
-// Prompt portions (ragged rows, any length), in blocks of four tokens: three launches.
+// Prompt portions (ragged rows, any length): three launches, the first two those of cdelta_chunk.cu where a chunk scratch is given (bf16 models), else,
+// in blocks of four tokens:
 //   prep   decays, unit keys and removal rates, and per block everything that does not depend on the state.  W2 tanh(l) of sixteen
 //          tokens is a product on the tensor cores: W2 is bf16, tanh(l) enters as three bf16 parts (24 bits), sums are fp32
 //   scan   the recurrence.  Columns of the state are independent, so a warp owns eight value columns for the whole portion: eight
@@ -705,6 +706,10 @@ static int cdelta_go(const CdeltaParams& p, bool single, cudaStream_t stream) {
     const int smem = ((5 + kCdParts) * DP + cd_rank_pad(p.rank) + 2 * p.VP) * 4;
     return static_cast<int>(launch(cdelta_step_kernel<NI>, dim3(p.H, p.nseq), dim3(32 * warps), smem, stream, 2, p));
   }
+  if (p.chunk != nullptr) {
+    const int r = saber_cdelta_chunk_launch(&p, stream);
+    return r != 0 ? r : static_cast<int>(launch(cdelta_out_kernel, dim3(p.M, (p.H + 7) / 8), dim3(256), 0, stream, 0, p));
+  }
   static bool ready[64];
   constexpr int smem = kCdStages * (cd_words(DP) + kCdVWords) * 4;
   cudaError_t e = cd_allow(cdelta_scan_kernel<NI>, ready, smem);
@@ -728,7 +733,7 @@ extern "C" int saber_cdelta_launches(int single_row) { return single_row ? 1 : 3
 extern "C" int saber_cdelta_launch(const saber::CdeltaParams* p, int single_row, cudaStream_t stream) {
   using namespace saber;
   if (p->M <= 0 || p->nseq <= 0 || p->H <= 0 || p->D < 1 || p->D > p->DP || p->D > p->VP || (p->VP & 7) || p->VP > 512 || p->rank < 1 || p->rank > 2048 ||
-      p->w2 == nullptr || p->state == nullptr || (!single_row && (p->rec == nullptr || p->vb == nullptr || p->o == nullptr)))
+      p->w2 == nullptr || p->state == nullptr || (!single_row && (p->o == nullptr || (p->chunk == nullptr && (p->rec == nullptr || p->vb == nullptr)))))
     return static_cast<int>(cudaErrorInvalidValue);
   switch (p->DP) {
     case 64: return cdelta_go<1>(*p, single_row != 0, stream);

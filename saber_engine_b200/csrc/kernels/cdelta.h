@@ -31,9 +31,13 @@ struct CdeltaParams {
   int M, nseq, H, D, DP, VP, n_slots;
   float eps, unit_eps, out_scale;
   uint32_t* err;
+  float* chunk;               // scratch of saber_cdelta_chunk_floats: prompt portions go sixteen tokens at a time on the tensor cores; null: the scan
 };
 
 }  // namespace saber
 
+// Scratch of the chunk form in floats (0: it does not take these sizes), and its first two launches (cdelta_chunk.cu)
+extern "C" size_t saber_cdelta_chunk_floats(const saber::CdeltaParams* p);
+int saber_cdelta_chunk_launch(const saber::CdeltaParams* p, cudaStream_t stream);
 extern "C" int saber_cdelta_launches(int single_row);
 extern "C" int saber_cdelta_launch(const saber::CdeltaParams* p, int single_row, cudaStream_t stream);

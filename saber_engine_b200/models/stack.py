@@ -467,7 +467,7 @@ class StackModel:
         mx = lambda it: max(it, default=0)    # noqa: E731
         wk = {"splits": self._splits(M, decode)}
         if not decode:
-            floats = {id(m): self._chunk_floats(m, M, nseq) for m in ms if isinstance(m, (DeltaMixer, OuterMixer))}
+            floats = {id(m): self._chunk_floats(m, M, nseq) for m in ms if isinstance(m, (DeltaMixer, OuterMixer, ChannelDeltaMixer))}
             scan = [m for m in de if not floats.get(id(m))]
             blk = M // 4 + nseq                           # blocks of four tokens
             wk["kq"] = f32(blk * mx(m.kv_heads * (8 * m.dim_pad + 16) for m in scan))
@@ -478,9 +478,9 @@ class StackModel:
             wk["o"] = f32(M * mx(m.heads * m.vdim_pad for m in outer))
         cd, conv = [m for m in ms if isinstance(m, ChannelDeltaMixer)], [m for m in gr if m.taps]
         if cd and not decode:
-            blk = M // 4 + nseq
-            wk["cd_rec"] = f32(blk * mx(m.heads * (17 * m.dim_pad + 64) for m in cd))
-            wk["cd_v"] = f32(blk * mx(m.heads * ((m.vdim_pad + 31) // 32) * 128 for m in cd))
+            blk, by_four = M // 4 + nseq, [m for m in cd if not floats[id(m)]]
+            wk["cd_rec"] = f32(blk * mx(m.heads * (17 * m.dim_pad + 64) for m in by_four))
+            wk["cd_v"] = f32(blk * mx(m.heads * ((m.vdim_pad + 31) // 32) * 128 for m in by_four))
             wk["cd_o"] = f32(M * mx(m.heads * m.vdim_pad for m in cd))
         if conv:
             wk["conv_x"], wk["conv_ss"] = f32(M * mx(self._conv_width(m) for m in conv)), f32(M * mx(self._conv_parts(m) for m in conv))
@@ -526,6 +526,10 @@ class StackModel:
             p = N.DeltaParams()
             p.M, p.nseq, p.H, p.HK, p.DP, p.VP = M, nseq, m.heads, m.kv_heads, m.dim_pad, m.vdim_pad
             return N.lib().saber_delta_chunk_floats(C.byref(p))
+        if isinstance(m, ChannelDeltaMixer):
+            p = N.CdeltaParams()
+            p.M, p.nseq, p.H, p.DP, p.VP, p.rank = M, nseq, m.heads, m.dim_pad, m.vdim_pad, m.rank
+            return N.lib().saber_cdelta_chunk_floats(C.byref(p))
         p = N.SsdParams()
         p.M, p.nseq, p.H, p.HK, p.N, p.DP, p.V, p.VP, p.taps = M, nseq, m.heads, m.kv_heads, m.dim, m.dim_pad, m.vdim, m.vdim_pad, m.taps
         return N.lib().saber_ssd_chunk_floats(C.byref(p))
@@ -582,6 +586,8 @@ class StackModel:
         p.w2, p.w2_f32, p.rank, p.w0, p.norm_w = x["w2"].data_ptr(), int(self.f32), m.rank, x["w0"].data_ptr(), x["norm"].data_ptr()
         p.state = self.state[key].data_ptr()
         p.rec, p.vb, p.o = (N.ptr(wk.get(k)) for k in ("cd_rec", "cd_v", "cd_o"))
+        if "chunk" in wk and self._chunk_floats(m, M, nseq):
+            p.chunk = wk["chunk"].data_ptr()
         p.cu_rows, p.slots, p.pos = at(lay.cu_rows), at(lay.slots), at(lay.pos)
         p.out, p.out_k0, p.out_scale, p.M, p.nseq = m_op, k0, scale, M, nseq
         p.H, p.D, p.DP, p.VP, p.n_slots = m.heads, m.dim, m.dim_pad, m.vdim_pad, self.n_slots

@@ -692,8 +692,9 @@ class StackConfig:
         """Scratch of the prompt scans of delta rules and of convolved queries, keys and values (one layer at a time)."""
         n = [0]
         for m in self.mixers():
-            if isinstance(m, ChannelDeltaMixer):
-                n.append(m.heads * (17 * m.dim_pad + 64 + 4 * m.vdim_pad + 128) // 4 + m.heads * m.vdim_pad)
+            if isinstance(m, ChannelDeltaMixer):         # (blocks of four tokens in fp32 rows, or of sixteen in bf16 parts)
+                slices = (m.vdim_pad + 31) // 32
+                n.append(max(m.heads * (17 * m.dim_pad + 64 + 4 * m.vdim_pad + 128) // 4, m.heads * (388 * m.dim_pad + 9216 + 2304 * slices) // 64) + m.heads * m.vdim_pad)
             elif isinstance(m, DeltaMixer):
                 slices = (m.vdim_pad + 31) // 32
                 n.append((m.kv_heads * 192 * m.dim_pad + m.heads * (2304 * slices + 4864)) // 64 + m.heads * m.vdim_pad)

@@ -239,7 +239,7 @@ class CdeltaParams(C.Structure):
     _fields_ = [("x", P), ("ldx", I), ("r_off", I), ("k_off", I), ("v_off", I), ("a_off", I), ("l_off", I), ("g_off", I), ("w2", P), ("w2_f32", I),
                 ("rank", I), ("w0", P), ("norm_w", P), ("state", P), ("rec", P), ("vb", P), ("o", P), ("cu_rows", P), ("slots", P), ("pos", P),
                 ("out", Operand), ("out_k0", I), ("M", I), ("nseq", I), ("H", I), ("D", I), ("DP", I), ("VP", I), ("n_slots", I), ("eps", F),
-                ("unit_eps", F), ("out_scale", F), ("err", P)]
+                ("unit_eps", F), ("out_scale", F), ("err", P), ("chunk", P)]
 
 
 class JoinParams(C.Structure):
@@ -384,6 +384,7 @@ def _declare(L: C.CDLL) -> None:
         "saber_ssd_launch": (I, [C.POINTER(SsdParams), I, S]),
         "saber_ssd_chunk_floats": (C.c_size_t, [C.POINTER(SsdParams)]),
         "saber_delta_chunk_floats": (C.c_size_t, [C.POINTER(DeltaParams)]),
+        "saber_cdelta_chunk_floats": (C.c_size_t, [C.POINTER(CdeltaParams)]),
         "saber_gqa_form": (I, [C.POINTER(GqaParams)]),
         "saber_gqa_launch": (I, [C.POINTER(GqaParams), S]),
         "saber_cdelta_launch": (I, [C.POINTER(CdeltaParams), I, S]),

@@ -108,3 +108,52 @@ def test_delta_rule(H, HK, D, V, gate, pieces):
         _near(torch.cat(got[j]), torch.stack(want))
         _near(state[j + 1, :, :V, :D].transpose(1, 2), S)
     assert not state[0].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pieces", PIECES)
+@pytest.mark.parametrize("H,D,rank", [(5, 128, 96), (4, 64, 16), (3, 72, 256), (9, 20, 33)])
+def test_channel_delta_rule(H, D, rank, pieces):
+    lens = [sum(p[j] for p in pieces) for j in range(4)]
+    DP, VP, g = (D + 63) // 64 * 64, (D + 7) // 8 * 8, torch.Generator(device=DEV).manual_seed(H + D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)                  # noqa: E731
+    off, ld = _offsets((("r", H * D), ("k", H * D), ("v", H * D), ("a", H * D), ("l", rank), ("g", H * D)))
+    x, w2 = [rnd(n, ld) for n in lens], (rnd(H * D, rank) * rank ** -0.5).bfloat16()
+    w0, nw = torch.rand(H * D, generator=g, device=DEV) * 6 - 5, torch.ones(H * D, device=DEV)
+    w2_p = torch.zeros(H * D, (rank + 15) // 16 * 16, dtype=torch.bfloat16, device=DEV)
+    w2_p[:, :rank] = w2
+    state, err, got = _f32(5, H, VP, DP), _i32([0] * 4), [[] for _ in lens]
+
+    def launch(piece, done):
+        cu, slots, pos, at = _tables(piece, done)
+        M = at[-1]
+        xs, o, out = torch.cat([x[j][done[j]:done[j] + n] for j, n in enumerate(piece)]).contiguous(), _f32(M, H, VP), _f32(M, H * D)
+        p = N.CdeltaParams()
+        p.x, p.ldx = xs.data_ptr(), ld
+        p.r_off, p.k_off, p.v_off, p.a_off, p.l_off, p.g_off = (off[z] for z in "rkvalg")
+        p.w2, p.w2_f32, p.rank, p.w0, p.norm_w, p.state, p.o = w2_p.data_ptr(), 0, rank, w0.data_ptr(), nw.data_ptr(), state.data_ptr(), o.data_ptr()
+        p.cu_rows, p.slots, p.pos, p.out, p.out_scale, p.err = cu.data_ptr(), slots.data_ptr(), pos.data_ptr(), N.Operand(out.data_ptr(), M, H * D, 1), 1.0, err.data_ptr()
+        p.M, p.nseq, p.H, p.D, p.DP, p.VP, p.n_slots, p.eps, p.unit_eps = M, 4, H, D, DP, VP, 5, 1e-6, 1e-6
+        floats = N.lib().saber_cdelta_chunk_floats(C.byref(p))
+        assert floats > 0
+        scratch = torch.full((floats,), float("nan"), device=DEV)
+        p.chunk = scratch.data_ptr()
+        N.check(N.lib().saber_cdelta_launch(C.byref(p), 0, N.stream_handle()), "cdelta")
+        torch.cuda.synchronize()
+        assert int(err[0]) == 0
+        for j in range(4):
+            got[j].append(o[at[j]:at[j + 1], :, :D])
+    _portions(pieces, launch)
+    for j, n in enumerate(lens):
+        X = x[j].double()
+        r, k, v, a = (X[:, off[z]:off[z] + H * D].view(n, H, D) for z in "rkva")
+        low = torch.tanh(X[:, off["l"]:off["l"] + rank]) @ w2.double().T + w0.double()
+        dec, u = torch.exp(-math.exp(-0.5) * torch.sigmoid(low)).view(n, H, D), k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+        S, want = torch.zeros(H, D, D, dtype=torch.float64, device=DEV), []
+        for t in range(n):
+            held = torch.einsum("hd,hdv->hv", u[t], S)
+            S = dec[t][..., None] * S - (torch.sigmoid(a[t]) * u[t])[..., None] * held[:, None] + k[t][..., None] * v[t][:, None]
+            want.append(torch.einsum("hdv,hd->hv", S, r[t]))
+        _near(torch.cat(got[j]), torch.stack(want))
+        _near(state[j + 1, :, :D, :D].transpose(1, 2), S)
+    assert not state[0].any()
