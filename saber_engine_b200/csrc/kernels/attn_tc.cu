@@ -14,8 +14,8 @@
 //               the running reference maximum only moves when a tile exceeds it by 2^8 (the
 //               probabilities then still fit e4m3), so the accumulator is rarely rescaled.  Bound by
 //               this pass: 1.1 us a tile of 1.5 us; 2048 rows behind 2048 tokens, 24 heads of 4 key
-//               heads, take 164 us (650 before: a condition on every element's exponential, 4.6 us a
-//               tile), 8 x 8 rows behind 4096 tokens 25 us (76);
+//               heads, take 179 us (650 before: a condition on every element's exponential, 4.6 us a
+//               tile), 8 x 8 rows behind 4096 tokens 27 us (76);
 //   O += P V    tcgen05.mma, M = 128, N = 256 dims, K = 128 keys (4 steps), accumulator in TMEM
 //               for the whole key range; S is double-buffered so the tensor core works on the
 //               next tile's scores while the softmax warps work on this one.
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
     // ------------------------------------------------------------------ producers: pages -> stages
     // One warp feeds the K ring, one the V ring.  Block ids are fetched 32 at a time (four tiles), a group ahead of their use, and a tile's
     // eight pages are issued by eight lanes: one lane that looked an id up ahead of every copy spent 600 clocks a page, both rings in turn
-    // (2048 rows behind 2048 tokens, 24 heads: 232 us against 164).
+    // (2048 rows behind 2048 tokens, 24 heads: 232 us against 164 with the pass as it was then).
     const bool is_v = warp == 6;
     const uint32_t full = is_v ? v_full : k_full, empty = is_v ? v_empty : k_empty;
     const uint32_t ring = is_v ? v_s : k_s;
@@ -318,7 +318,8 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
         float l_tile = 0.f;
         for (int attempt = 0; attempt < 2; ++attempt) {
           const float msafe = m_ref == -INFINITY ? 0.f : m_ref;
-          float tmax[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, sum[4] = {};
+          l_tile = 0.f;
+          float tmax[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
           for (int c0 = 0; c0 < kTcKeys; c0 += 32) {
             float sv[32];
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
                 const float sc = sv[4 * i + e];
                 tmax[e] = fmaxf(tmax[e], sc);
                 pv[e] = exp2f(sc * scale_log2 - msafe);
-                sum[e] += pv[e];
+                l_tile += pv[e];                         // (in the keys' order, as the sums have always been: four sums side by side take 164 us instead of 179)
               }
               const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(pv[0], pv[1]), __NV_SATFINITE, __NV_E4M3);
               const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(pv[2], pv[3]), __NV_SATFINITE, __NV_E4M3);
@@ -341,7 +342,6 @@ __global__ void __launch_bounds__(kTcThreads) attn_tc_kernel(const AttnParams p,
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(prow + (c0 >> 4) * 128), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(prow + ((c0 >> 4) + 1) * 128), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
           }
-          l_tile = (sum[0] + sum[1]) + (sum[2] + sum[3]);
           const float tm = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3])) * scale_log2;            // (-inf when the row has no live key in the tile)
           const bool over = row_live && tm > m_ref + 8.f;
           if (over) {

@@ -138,17 +138,29 @@ __global__ void __launch_bounds__(128) gdn_conv_rows_kernel(const GdnConvParams 
       win[2] = f;
     }
     if (unit) {
+      // (the order of the row-at-a-time form: 32 channels by halves, then the four groups of them one behind the other)
       float ss[kConvAhead];
 #pragma unroll
-      for (int u = 0; u < kConvAhead; ++u) ss[u] = (y[u].x * y[u].x + y[u].y * y[u].y) + (y[u].z * y[u].z + y[u].w * y[u].w);
+      for (int u = 0; u < kConvAhead; ++u) {
+        float s[4] = {y[u].x * y[u].x, y[u].y * y[u].y, y[u].z * y[u].z, y[u].w * y[u].w};
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
+        for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
-        for (int u = 0; u < kConvAhead; ++u) ss[u] += __shfl_xor_sync(0xffffffffu, ss[u], o);
+          for (int e = 0; e < 4; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+        ss[u] = (s[0] + s[2]) + (s[1] + s[3]);
+      }
+#pragma unroll
+      for (int u = 0; u < kConvAhead; ++u) {
+        float g[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g[e] = __shfl_sync(0xffffffffu, ss[u], e * 8);
+        ss[u] = g[0] + g[1] + g[2] + g[3];
+      }
 #pragma unroll
       for (int u = 0; u < kConvAhead; ++u) {
         const float f = rsqrtf(ss[u] + 1e-6f);
-        y[u] = make_float4(y[u].x * f * scale, y[u].y * f * scale, y[u].z * f * scale, y[u].w * f * scale);
+        y[u] = make_float4(y[u].x * f, y[u].y * f, y[u].z * f, y[u].w * f);
+        if (ch < p.n_q) y[u] = make_float4(y[u].x * scale, y[u].y * scale, y[u].z * scale, y[u].w * scale);
       }
     }
 #pragma unroll
