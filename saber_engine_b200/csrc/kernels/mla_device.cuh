@@ -72,4 +72,6 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // mla_mma.cu: the bf16 forms on the tensor cores
 int saber_mla_decode_attn(const saber::MlaParams* p, cudaStream_t stream);
 int saber_mla_expand_attn(const saber::MlaParams* p, cudaStream_t stream);
+bool saber_mla_expand_tc_ok(const saber::MlaParams* p);
+int saber_mla_expand_tc(const saber::MlaParams* p, cudaStream_t stream);
 bool saber_mla_decode_ok(const saber::MlaParams* p);
