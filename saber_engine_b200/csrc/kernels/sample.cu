@@ -38,30 +38,57 @@ __device__ __forceinline__ float key_logit(uint32_t key, float) {
   return __uint_as_float((key & 0x80000000u) ? (key & 0x7FFFFFFFu) : ~key);
 }
 
-// grid = rows, block 1024. out_idx[r] = argmax (global id = local + id_offset), out_val[r] = value.
+// Logits of a row that one 16-byte piece holds
+template <typename T> constexpr int kPiece = 16 / static_cast<int>(sizeof(T));
+__device__ __forceinline__ void piece_f(const uint4& u, float (&f)[8]) {          // bf16
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 x = __bfloat1622float2(h[i]);
+    f[2 * i] = x.x;
+    f[2 * i + 1] = x.y;
+  }
+}
+__device__ __forceinline__ void piece_f(const uint4& u, float (&f)[4]) {
+  f[0] = __uint_as_float(u.x);
+  f[1] = __uint_as_float(u.y);
+  f[2] = __uint_as_float(u.z);
+  f[3] = __uint_as_float(u.w);
+}
+
+// grid (kArgCtas, rows), a cluster per row: out_idx[r] = argmax (global id = local + id_offset), out_val[r] = value.  One CTA walking a
+// row is a chain of memory round trips (64 of them for 65,536 fp32 logits: 54 us); eight CTAs with four loads in flight a thread
+// meet in the first one's shared memory.
+constexpr int kArgCtas = 8, kArgLoads = 4;
 template <typename T>
-__global__ void __launch_bounds__(1024) argmax_kernel(const T* logits, int ld, int V,
-                                                      int id_offset, int32_t* out_idx,
-                                                      float* out_val) {
+__global__ void __cluster_dims__(kArgCtas, 1, 1) __launch_bounds__(512) argmax_kernel(const T* logits, int ld, int V,
+                                                                                      int id_offset, int32_t* out_idx,
+                                                                                      float* out_val) {
   pdl_wait();
-  __shared__ float sv[32];
-  __shared__ int si[32];
-  const int r = blockIdx.x;
+  __shared__ float sv[16], cv[kArgCtas];
+  __shared__ int si[16], ci[kArgCtas];
+  constexpr int P = kPiece<T>;
+  const int r = blockIdx.y, rank = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const T* row = logits + static_cast<size_t>(r) * ld;
   float bv = -INFINITY;
   int bi = V;  // "cols" when nothing finite/non-NaN was seen
-  const int nvec = sizeof(T) == 2 ? V >> 3 : 0;
-  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(row + v * 8);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const int pieces = (reinterpret_cast<uintptr_t>(logits) & 15) == 0 ? V / P : 0, per = (pieces + kArgCtas - 1) / kArgCtas, end = min(pieces, (rank + 1) * per);
+  for (int v0 = rank * per + threadIdx.x; v0 < end; v0 += 512 * kArgLoads) {
+    uint4 raw[kArgLoads];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __bfloat1622float2(h[i]);
-      if (f.x == f.x && better(f.x, v * 8 + 2 * i, bv, bi)) { bv = f.x; bi = v * 8 + 2 * i; }
-      if (f.y == f.y && better(f.y, v * 8 + 2 * i + 1, bv, bi)) { bv = f.y; bi = v * 8 + 2 * i + 1; }
-    }
+    for (int u = 0; u < kArgLoads; ++u)
+      if (v0 + 512 * u < end) raw[u] = *reinterpret_cast<const uint4*>(row + static_cast<size_t>(v0 + 512 * u) * P);
+#pragma unroll
+    for (int u = 0; u < kArgLoads; ++u)
+      if (v0 + 512 * u < end) {
+        float f[P];
+        piece_f(raw[u], f);
+#pragma unroll
+        for (int i = 0; i < P; ++i)
+          if (f[i] == f[i] && better(f[i], (v0 + 512 * u) * P + i, bv, bi)) { bv = f[i]; bi = (v0 + 512 * u) * P + i; }
+      }
   }
-  for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) {
+  for (int i = pieces * P + rank * 512 + threadIdx.x; i < V; i += 512 * kArgCtas) {
     const float f = logit_f(row[i]);
     if (f == f && better(f, i, bv, bi)) { bv = f; bi = i; }
   }
@@ -71,22 +98,36 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const T* logits, int ld, i
     const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
     if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) { sv[warp] = bv; si[warp] = bi; }
   __syncthreads();
   if (warp == 0) {
-    bv = lane < (blockDim.x >> 5) ? sv[lane] : -INFINITY;
-    bi = lane < (blockDim.x >> 5) ? si[lane] : V;
+    bv = lane < 16 ? sv[lane] : -INFINITY;
+    bi = lane < 16 ? si[lane] : V;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
       const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
     }
-    if (lane == 0) {
-      out_idx[r] = bi + id_offset;
-      if (out_val) out_val[r] = bv;
+    if (lane == 0) {                               // into the first CTA of the cluster
+      const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(&cv[rank])), b = static_cast<uint32_t>(__cvta_generic_to_shared(&ci[rank]));
+      asm volatile(
+          "{\n\t.reg .b32 x, y;\n\t"
+          "mapa.shared::cluster.u32 x, %0, 0;\n\t"
+          "mapa.shared::cluster.u32 y, %1, 0;\n\t"
+          "st.shared::cluster.f32 [x], %2;\n\t"
+          "st.shared::cluster.b32 [y], %3;\n\t}\n" ::"r"(a), "r"(b), "f"(bv), "r"(bi) : "memory");
     }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank == 0 && threadIdx.x == 0) {
+    bv = cv[0];
+    bi = ci[0];
+#pragma unroll
+    for (int i = 1; i < kArgCtas; ++i)
+      if (better(cv[i], ci[i], bv, bi)) { bv = cv[i]; bi = ci[i]; }
+    out_idx[r] = bi + id_offset;
+    if (out_val) out_val[r] = bv;
   }
 }
 
@@ -263,10 +304,10 @@ extern "C" int saber_argmax_launch(const void* logits, int f32, int rows, int ld
   if (rows <= 0) return 0;
   if (ld & 7) return static_cast<int>(cudaErrorInvalidValue);
   if (f32)
-    saber::launch(saber::argmax_kernel<float>, dim3(rows), dim3(1024), 0, stream, 0, static_cast<const float*>(logits), ld, V, id_offset,
+    saber::launch(saber::argmax_kernel<float>, dim3(saber::kArgCtas, rows), dim3(512), 0, stream, 0, static_cast<const float*>(logits), ld, V, id_offset,
                   out_idx, out_val);
   else
-    saber::launch(saber::argmax_kernel<__nv_bfloat16>, dim3(rows), dim3(1024), 0, stream, 0, static_cast<const __nv_bfloat16*>(logits), ld, V,
+    saber::launch(saber::argmax_kernel<__nv_bfloat16>, dim3(saber::kArgCtas, rows), dim3(512), 0, stream, 0, static_cast<const __nv_bfloat16*>(logits), ld, V,
                   id_offset, out_idx, out_val);
   return static_cast<int>(cudaGetLastError());
 }
