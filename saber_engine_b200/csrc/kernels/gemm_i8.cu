@@ -57,12 +57,6 @@ constexpr int kUBufs = 3;                // W4: widened int8 operand buffers (tr
                                          // the buffer-free round trip overlap with three)
 
 // GELU of a rounded linear output: tanh form (x * 0.5 * (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3)))) or erf form.
-__device__ __forceinline__ float gelu_f(float x, bool erf_form) {
-  if (erf_form) return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-  return 0.5f * x * (1.f + tanhf(u));
-}
-
 // Grid-wide barrier for grids that are resident as a whole (one CTA per SM, grid <= SM count).  ONE
 // thread per CTA calls, after a CTA-level barrier that ordered the other threads' writes before it.
 // `ctr` is zero when the kernel starts.  The wait is bounded like every other wait here: when it
@@ -92,13 +86,11 @@ __device__ __forceinline__ void grid_depart(uint32_t* ctr, uint32_t n_ctas) {
 // two operand buffers instead of three, at most 102 registers -- so that TWO CTAs share an SM: an
 // expert tile is only 16 k-blocks long, and the second CTA's main loop hides the first one's
 // start-up latency (cold weights: 3-4 us to the first MMA) and epilogue.
-// kBf: the bf16 x bf16 instantiation (optional scales, bias, activation / residual epilogue); the
-// integer and MXFP4 instantiations compile none of it.
 // kFp4: native block-scaled FP4 x FP4 (tcgen05.mma kind::mxf4nvf4 / kind::mxf4): both operands stay
 // packed e2m1 in shared memory (a 32 KiB stage is 256 features x 256 k), their block scales ride
 // behind the tiles, are copied into tensor memory by tcgen05.cp and applied by the tensor core; no
 // transform warps, fp32 accumulators, the per-token and per-tensor scales in the epilogue.
-template <bool kLean, bool kBf = false, bool kFp4 = false>
+template <bool kLean, bool kFp4 = false>
 __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int stages, const RowOpParams* tail) {
   const int nub = (kLean || p.mtiles == 2) ? 2 : kUBufs;     // operand buffers in use
   extern __shared__ uint8_t smem_raw[];
@@ -107,7 +99,6 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
   __shared__ uint32_t is_last_s;
   __shared__ uint32_t abort_s;
   __shared__ float w_scale_s[256];
-  __shared__ float bias_s[kBf ? 256 : 1];
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -127,7 +118,7 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
   // the few SMs it leaves free.
   // half tiles (p.halves == 2): two CTAs share a packed weight tile, each widens and multiplies only
   // its 128 rows of it (the low or the high nibbles) -- twice the CTAs without split-K
-  const int halves = (!kLean && !kBf && p.halves == 2) ? 2 : 1;
+  const int halves = (!kLean && p.halves == 2) ? 2 : 1;
   // Two token tiles per CTA (long row runs): the grid is (token tile pairs, feature tiles), so CTAs that are
   // scheduled together share a weight tile -- it comes from memory once and from L2 for the other row tiles
   // (with the feature tile running fastest every row-tile wave would stream the whole weight again).
@@ -163,9 +154,8 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
   const int n0 = tile_n * 256 + half * 128;
   // weight formats: 0 = int8 tiles, 1 = packed int4, 2 = MXFP4 (packed e2m1 + 1 KiB of block shifts)
   // 3 = bf16 x bf16: both operands pass through like int8 tiles (K counted in bytes), fp32 accumulators
-  const bool mx = !kBf && !kFp4 && p.w4 == 2;
-  constexpr bool bf = kBf;
-  const bool widen = !kBf && !kFp4 && p.w4 != 0;
+  const bool mx = !kFp4 && p.w4 == 2;
+  const bool widen = !kFp4 && p.w4 != 0;
   // FP4: w4 = 4 is NVFP4 (e4m3 scale per 16 values: 16 scales per row and k-block), 5 is MXFP4 (e8m0 per 32: 8).
   // Scales are stored as 512-byte atoms (128 rows x 4 scales, byte (r % 32) * 16 + (r / 32) * 4 + s):
   // the shape tcgen05.cp moves into four tensor-memory columns.
@@ -306,7 +296,6 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
     if (lane == 0) {
       // M = 128 token rows (only the first nt are real), N = 256 output features
       const uint32_t idesc = mx ? make_idesc(kCFmtF32, kFmtE4M3, kFmtE4M3, 128, 256)
-                           : bf ? make_idesc(kCFmtF32, kFmtBF16, kFmtBF16, 128, 256)
                                 : make_idesc(kCFmtS32, kFmtS8, kFmtS8, 128, halves == 2 ? 128 : 256);
       const uint64_t desc_hi = make_desc_k128(0);  // everything but the start address
       uint32_t a_addr = a_smem;
@@ -354,11 +343,6 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
             mma_f8_ss(dj, aj + 2, b_desc + 2, idesc, 1u);
             mma_f8_ss(dj, aj + 4, b_desc + 4, idesc, 1u);
             mma_f8_ss(dj, aj + 6, b_desc + 6, idesc, 1u);
-          } else if (bf) {   // 16 bf16 = 32 bytes along K per instruction: the same +2 steps
-            mma_f16_ss(dj, aj, b_desc, idesc, it != 0 ? 1u : 0u);
-            mma_f16_ss(dj, aj + 2, b_desc + 2, idesc, 1u);
-            mma_f16_ss(dj, aj + 4, b_desc + 4, idesc, 1u);
-            mma_f16_ss(dj, aj + 6, b_desc + 6, idesc, 1u);
           } else {
             mma_i8_ss(dj, aj, b_desc, idesc, it != 0 ? 1u : 0u);
             mma_i8_ss(dj, aj + 2, b_desc + 2, idesc, 1u);
@@ -379,7 +363,7 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
       // CTA gives its tensor memory back (the status word already tells the host the result is void).
       if (!ok) mbar_wait(bar_acc, 0, nullptr, 0);
       SABER_STAMP(6);
-    } else if (!kLean && !kBf && p.tail_mode == 1 && blockIdx.x == 0 && blockIdx.y == 0) {
+    } else if (!kLean && p.tail_mode == 1 && blockIdx.x == 0 && blockIdx.y == 0) {
       // in-tile silu * mul + quant: the row maxima start from zero; this launch's first CTA cleans
       // them here (the previous user finished with its whole grid) and raises the "clean" flag
       pdl_wait();
@@ -388,7 +372,7 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
       __syncwarp(0xFFFFFFFEu);
       if (lane == 1)
         asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.tail_sync + kTailFlagsAt + 255), "r"(1u) : "memory");
-    } else if (!kLean && !kBf && p.tail_mode == 3 && split == 0) {
+    } else if (!kLean && p.tail_mode == 3 && split == 0) {
       // Row tail on the accumulator blocks: nobody re-zeroes a block after reading it (16-byte
       // zero stores from one CTA per row share sectors across CTAs and are ruinously slow), so the
       // first split of every tile cleans its block HERE, in whole lines, while the pipeline
@@ -412,14 +396,7 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
     const int q4 = warp & 3;                     // TMEM lane quarter this warp may access
     bool ok = true;
     if (tgroup == 0) {  // epilogue warps stage the per-feature scales while the pipeline fills
-      if constexpr (kBf) {
-        for (int j = tid_t; j < 256; j += 128) {
-          w_scale_s[j] = (n0 + j < p.N) ? (p.w_scale ? w_scale_base[n0 + j] : 1.f) : 0.f;
-          bias_s[j] = (p.bias && n0 + j < p.N) ? p.bias[n0 + j] : 0.f;
-        }
-      } else {
-        for (int j = tid_t; j < 256; j += 128) w_scale_s[j] = (n0 + j < p.N) ? w_scale_base[n0 + j] : 0.f;
-      }
+      for (int j = tid_t; j < 256; j += 128) w_scale_s[j] = (n0 + j < p.N) ? w_scale_base[n0 + j] : 0.f;
     }
     if (widen) {
       // The two groups of four warps take the k-blocks in turn (group g: blocks g, g + 2, ...).  A
@@ -525,8 +502,8 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
     // wide forms: both groups read the accumulator out (half of the columns each: either group's
     // four warps cover the four TMEM lane quarters) -- the in-tile silu * mul + quant and the
     // staging of split-K partial sums for the bulk reduction
-    const bool bulk = !kLean && !kBf && !kFp4 && !mx && p.splits > 1 && p.acc != nullptr;
-    const bool smq = !kLean && !kBf && p.tail_mode == 1;
+    const bool bulk = !kLean && !kFp4 && !mx && p.splits > 1 && p.acc != nullptr;
+    const bool smq = !kLean && p.tail_mode == 1;
     const bool wide = bulk || smq;
     if (tgroup == 0 || pair || wide) {
       // the epilogue warps decide TOGETHER whether to run the epilogue: the named barriers
@@ -538,7 +515,7 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
     } else {
       ok = false;  // only the first group (TMEM lane quarters 2,3,0,1) is the epilogue
     }
-    if constexpr (!kLean && !kBf) {
+    if constexpr (!kLean) {
       if (bulk) {
         // split-K partial sums: the live rows go to shared memory as [c4][nt rows][4 ints] (a warp's
         // 32 rows store 512 contiguous bytes), rows between the live count and nt as zeros
@@ -704,7 +681,7 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
       const int ncols = halves == 2 ? 128 : min(256, p.N_pad - n0);
       // accumulator words are int32 (integer formats) or fp32 bits (MXFP4)
       auto acc_f = [&](uint32_t raw) -> float {
-        return (mx || bf || kFp4) ? __uint_as_float(raw) : static_cast<float>(static_cast<int32_t>(raw));
+        return (mx || kFp4) ? __uint_as_float(raw) : static_cast<float>(static_cast<int32_t>(raw));
       };
       // tensor-parallel mode: a finished 16-byte group of outputs goes to every rank's receive
       // region (slot = parity of the call's sequence number, source = this rank)
@@ -751,7 +728,7 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
         if (!kLean && p.tp_rpr > 0) tp_owner = mb / p.tp_rpr;
         if (j2 > j2_lo) named_bar_sync(ebar, 128);   // the staging buffer is free again
         if (warp_livej) {
-          const float asc = livej ? ((!kBf || p.a_scale) ? p.a_scale[mb + row] : 1.f) : 0.f;
+          const float asc = livej ? p.a_scale[mb + row] : 0.f;
           for (int c = 0; c < ncols; c += 32) {
             uint32_t r[32];
             tmem_ld32(tl + c, r);
@@ -760,16 +737,9 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
               uint32_t pk[16];
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
-                float lo = acc_f(r[2 * j]) * (asc * w_scale_s[c + 2 * j]);
-                float hi = acc_f(r[2 * j + 1]) * (asc * w_scale_s[c + 2 * j + 1]);
-                if constexpr (kBf) { lo += bias_s[c + 2 * j]; hi += bias_s[c + 2 * j + 1]; }
-                __nv_bfloat162 b2 = __floats2bfloat162_rn(lo, hi);
-                if constexpr (kBf) {
-                  if (p.epi == 1 || p.epi == 2) {   // the activation works on the rounded linear output
-                    const float2 y = __bfloat1622float2(b2);
-                    b2 = __floats2bfloat162_rn(gelu_f(y.x, p.epi == 2), gelu_f(y.y, p.epi == 2));
-                  }
-                }
+                const float lo = acc_f(r[2 * j]) * (asc * w_scale_s[c + 2 * j]);
+                const float hi = acc_f(r[2 * j + 1]) * (asc * w_scale_s[c + 2 * j + 1]);
+                const __nv_bfloat162 b2 = __floats2bfloat162_rn(lo, hi);
                 pk[j] = *reinterpret_cast<const uint32_t*>(&b2);
               }
 #pragma unroll
@@ -795,19 +765,6 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
                          : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                          : "r"(stage_s + rw * 512 + (chunk << 4)));
             if (!col_ok || col >= ncols) continue;
-            if (kBf && p.epi == 3 && p.res != nullptr) {     // residual add on the rounded linear output
-              const __nv_bfloat16* rp = p.res + static_cast<size_t>(mb + rw) * p.ldo + n0 + col;
-              __nv_bfloat16* pv = reinterpret_cast<__nv_bfloat16*>(&v);
-              if (full) {
-                const uint4 rv = *reinterpret_cast<const uint4*>(rp);
-                const __nv_bfloat16* pr = reinterpret_cast<const __nv_bfloat16*>(&rv);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) pv[j] = __float2bfloat16(__bfloat162float(pv[j]) + __bfloat162float(pr[j]));
-              } else {
-                for (int j = 0; j < 8; ++j)
-                  if (n0 + col + j < p.N) pv[j] = __float2bfloat16(__bfloat162float(pv[j]) + __bfloat162float(rp[j]));
-              }
-            }
             if (tp) {
               tp_push16(mb + rw, n0 + col, v);
             } else if (full) {
@@ -1048,7 +1005,7 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_d, kTmemCols);
   if (threadIdx.x == 32) SABER_STAMP(9);
-  if constexpr (!kLean && !kBf) {
+  if constexpr (!kLean) {
     if ((p.tail_mode == 2 || p.tail_mode == 3) && tail != nullptr) {
       // Row tail.  Every CTA arrives here whatever happened above (an aborted pipeline has set the
       // status word; the barrier still completes), then the rows are dealt round-robin to the CTAs.
@@ -1104,11 +1061,8 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_i8_tail_kernel(const GemmI8
                                                                     const __grid_constant__ RowOpParams tail) {
   gemm_i8_body<false>(p, stages, &tail);
 }
-__global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(const GemmI8Params p, const int stages) {
-  gemm_i8_body<false, true>(p, stages, nullptr);
-}
 __global__ void __launch_bounds__(kGemmThreads) gemm_fp4_kernel(const GemmI8Params p, const int stages) {
-  gemm_i8_body<false, false, true>(p, stages, nullptr);
+  gemm_i8_body<false, true>(p, stages, nullptr);
 }
 __global__ void __launch_bounds__(kGemmThreads, 2) gemm_i8_lean_kernel(const GemmI8Params p, const int stages) {
   gemm_i8_body<true>(p, stages, nullptr);
@@ -1130,7 +1084,6 @@ static int device_setup(int* sm_count) {
   if (sms[dev] == 0) {
     const int kSmemLimit = 224 * 1024;
     cudaFuncSetAttribute(gemm_i8_lean_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
-    cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     cudaFuncSetAttribute(gemm_fp4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     cudaFuncSetAttribute(gemm_i8_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     e = cudaFuncSetAttribute(gemm_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
@@ -1177,7 +1130,7 @@ extern "C" int saber_gemm_i8_launch(const saber::GemmI8Params* p, int stages, cu
   if (p->w4 == 4 || p->w4 == 5) {
     // native FP4: K counts values (256 per k-block); inside the kernel K counts the 128-byte rows of a block
     if ((p->K & 255) || p->a_sf == nullptr || p->group_tiles || p->tail_mode != 0 || p->tp_nranks > 1 || p->ag_flags != nullptr ||
-        p->halves == 2 || p->bias || p->epi || (p->M > 128 && p->nt != 128))
+        p->halves == 2 || (p->M > 128 && p->nt != 128))
       return static_cast<int>(cudaErrorInvalidValue);
     GemmI8Params q = *p;
     q.K = p->K >> 1;
@@ -1207,8 +1160,8 @@ extern "C" int saber_gemm_i8_launch(const saber::GemmI8Params* p, int stages, cu
   }
   const int kSmemLimit = 224 * 1024;  // opt-in maximum minus the kernel's static shared memory
   const bool widen_l = p->w4 == 1 || p->w4 == 2;
-  if (p->w4 < 0 || p->w4 > 3 || (p->w4 == 3 && (p->splits != 1 || p->group_tiles))) return static_cast<int>(cudaErrorInvalidValue);
-  if ((p->bias || p->epi) && p->w4 != 3) return static_cast<int>(cudaErrorInvalidValue);   // bias / activation / residual: bf16 mode only
+  if (p->w4 < 0 || p->w4 > 2) return static_cast<int>(cudaErrorInvalidValue);
+
   if (stages <= 0) stages = widen_l ? 8 : 5;   // one CTA per SM, as deep a ring as fits
   if (stages < 2) stages = 2;
   if (stages > kMaxStages) stages = kMaxStages;
@@ -1231,7 +1184,7 @@ extern "C" int saber_gemm_i8_launch(const saber::GemmI8Params* p, int stages, cu
   q.coop = (p->splits > 1 && p->coop >= 0 && resident) ? 1 : 0;
   if (p->tail_mode != 0) {
     // the tails wait for the whole grid: every CTA must be resident, one token-tile form only
-    if (!resident || p->group_tiles || p->w4 == 3 || p->tail_sync == nullptr || p->mtiles == 2 ||
+    if (!resident || p->group_tiles || p->tail_sync == nullptr || p->mtiles == 2 ||
         false)
       return static_cast<int>(cudaErrorInvalidValue);
     if (p->tail_mode == 1 &&
@@ -1270,7 +1223,7 @@ extern "C" int saber_gemm_i8_launch(const saber::GemmI8Params* p, int stages, cu
     if (smem2 <= kSmemLimit) {
       q.mtiles = 2;
       dim3 grid2((p->M + 255) / 256, p->N_pad / 256, 1);      // token tile pairs run fastest (see raster_m in the kernel)
-      return static_cast<int>(saber::launch(p->w4 == 3 ? gemm_bf16_kernel : gemm_i8_kernel, grid2, dim3(kGemmThreads), smem2, stream, 2, q, st2));
+      return static_cast<int>(saber::launch(gemm_i8_kernel, grid2, dim3(kGemmThreads), smem2, stream, 2, q, st2));
     }
   }
   // CTAs that wait for one another (split-K parts, tails) need the grid resident as a whole: it has
@@ -1296,7 +1249,7 @@ extern "C" int saber_gemm_i8_launch(const saber::GemmI8Params* p, int stages, cu
     }
     return static_cast<int>(saber::launch(gemm_i8_tail_kernel, grid, dim3(kGemmThreads), smem, stream, lflags, q, stages, tail));
   }
-  return static_cast<int>(saber::launch(p->w4 == 3 ? gemm_bf16_kernel : gemm_i8_kernel, grid, dim3(kGemmThreads), smem, stream, lflags, q, stages));
+  return static_cast<int>(saber::launch(gemm_i8_kernel, grid, dim3(kGemmThreads), smem, stream, lflags, q, stages));
 }
 
 extern "C" int saber_gemm_i8_tail_ok(const saber::GemmI8Params* p) {

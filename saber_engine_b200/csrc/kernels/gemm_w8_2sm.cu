@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(k2Threads, 1) gemm_w8_2sm_persistent_kernel(co
 extern "C" int saber_gemm_w8_2sm_ok(const saber::GemmI8Params* p) {
   return p->w4 == 0 && p->splits == 1 && p->M >= 512 && (p->M_pad % 512) == 0 && (p->K % 128) == 0 && (p->N_pad % 256) == 0 &&
                  (p->N % 8) == 0 && (p->ldo % 8) == 0 && p->tail_mode == 0 && p->tp_nranks <= 1 && p->ag_flags == nullptr &&
-                 p->group_tiles == nullptr && p->bias == nullptr && p->epi == 0 && p->halves != 2
+                 p->group_tiles == nullptr && p->halves != 2
              ? 1
              : 0;
 }

@@ -1,7 +1,7 @@
 // The vision tower's own kernels: rows -> bf16 GEMM operand (cast or LayerNorm, optional 4-row
 // grouping for the merger), the position-table gather, and non-causal attention with 2-D rotary
 // embedding.  The tower's linears (patch embed, qkv, proj, fc1 + GELU, fc2 + residual, merger) run on
-// the tcgen05 GEMM in its bf16 mode with bias / activation / residual in the epilogue.
+// vis_linear.cu with bias / activation / residual in the epilogue.
 //
 // Parity: the reference tower's op list and rounding points (crates/saber-kernels/hip/vision.hip:1-30):
 // every linear rounds to bf16 once and the activation / residual work on the rounded value;

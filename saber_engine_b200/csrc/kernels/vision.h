@@ -1,5 +1,4 @@
-// Launch interface of the vision tower's own kernels (the tower's linears run on the tcgen05 GEMM in
-// its bf16 mode, see gemm_i8.h).  Plain C types only.
+// Launch interface of the vision tower's kernels (vision.cu, vis_linear.cu).  Plain C types only.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
