@@ -153,7 +153,6 @@ __device__ __forceinline__ void gemm_i8_body(const GemmI8Params& p, const int st
   }
   const int n0 = tile_n * 256 + half * 128;
   // weight formats: 0 = int8 tiles, 1 = packed int4, 2 = MXFP4 (packed e2m1 + 1 KiB of block shifts)
-  // 3 = bf16 x bf16: both operands pass through like int8 tiles (K counted in bytes), fp32 accumulators
   const bool mx = !kFp4 && p.w4 == 2;
   const bool widen = !kFp4 && p.w4 != 0;
   // FP4: w4 = 4 is NVFP4 (e4m3 scale per 16 values: 16 scales per row and k-block), 5 is MXFP4 (e8m0 per 32: 8).

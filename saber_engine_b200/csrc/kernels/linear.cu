@@ -53,6 +53,12 @@ __device__ __forceinline__ float stored(const LinEpi& e, int n, float v) {      
 
 constexpr int kGatedTile = 248;           // features of a tile of act_kind 2; row 248 of the tile is their gate
 
+// Rows of the step.  (Without any, as in the walk ahead of a bucket's capture: all, so that every tile's path is taken.)
+__device__ __forceinline__ int live_rows(const LinParams& p) {
+  const int n = p.live != nullptr ? *p.live : 0;
+  return n > 0 ? min(p.M, n) : p.M;
+}
+
 // x[i] (eight stream values of rows m + 8 i, columns from n on) += the sum over the rows' routes of weight times expert row.  A lane holds
 // a route of each row; sixteen pieces of expert rows are requested together.
 __device__ __forceinline__ void add_routes(const LinEpi& e, int m, int rows, int n, bool cols, int lane, float4 (&x)[4][2]) {
@@ -296,6 +302,10 @@ __global__ void __launch_bounds__(kLinThreads, 1) lin_bf16_kernel(const __grid_c
     if (static_cast<int>(blockIdx.x) >= p.group_ntiles[0]) return;
     group = p.group_tiles[blockIdx.x];
   }
+  // A bucket's rows behind the step's own are padding: 1500 rows of a 2048-row bucket take 143 us a linear of Tepavik's on average, all 2048 took 179.  (The step's
+  // index tables are there before its first kernel starts.)
+  const int m_live = kGroup == 0 ? live_rows(p) : p.M;
+  if (kGroup == 0 && static_cast<int>(blockIdx.x) * p.nt * kMT >= m_live) return;
   __shared__ uint64_t bars[2 * kLinMaxStages + 1];
   __shared__ uint32_t tmem_base_s, is_last_s, abort_s;
   __shared__ float scale_s[256];
@@ -307,7 +317,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) lin_bf16_kernel(const __grid_c
   const int kb0 = split * kb_per;
   const int nkb = min(KB, kb0 + kb_per) - kb0;        // host guarantees >= 1
   const int m0 = kGroup != 0 ? group.y : tile_m * p.nt * kMT;
-  const int m_end = kGroup != 0 ? group.y + group.z : p.M;
+  const int m_end = kGroup != 0 ? group.y + group.z : m_live;
   const uint32_t abytes = static_cast<uint32_t>(p.nt) * 128u * kMT;
   const uint32_t a_smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t w_smem = a_smem + static_cast<uint32_t>(stages) * abytes;
@@ -339,7 +349,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) lin_bf16_kernel(const __grid_c
     // ---------------------------------------------------------------- producer
     if (lane == 0) {
       constexpr bool kCopyA = kGroup != 2;
-      const uint32_t acopy = kGroup == 0 ? abytes : static_cast<uint32_t>((group.z + 7) & ~7) * 128u;   // a group's own rows
+      const uint32_t acopy = kGroup == 0 ? (kMT == 2 && m0 + p.nt >= m_end ? abytes / 2 : abytes) : static_cast<uint32_t>((group.z + 7) & ~7) * 128u;   // a group's own rows
       const uint32_t tx = kLinTile + (kCopyA ? acopy : 0u);
       const uint64_t pol = gridDim.x > 1 ? l2_policy_evict_normal() : l2_policy_evict_first();
       const uint8_t* wp = static_cast<const uint8_t*>(p.w) + group.x * p.group_w_stride + (static_cast<size_t>(tile_n) * KB + kb0) * kLinTile;
@@ -392,7 +402,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) lin_bf16_kernel(const __grid_c
         const uint64_t b_desc = desc_hi | static_cast<uint64_t>((w_addr & 0x3FFFFu) >> 4);
 #pragma unroll
         for (int j2 = 0; j2 < kMT; ++j2) {
-          if (kGroup != 0 && j2 > 0 && j2 * p.nt >= group.z) break;
+          if (j2 > 0 && m0 + j2 * p.nt >= m_end) break;
           const uint32_t dj = tmem_d + static_cast<uint32_t>(j2) * 256u;
           const uint64_t aj = a_desc + static_cast<uint64_t>(j2) * (static_cast<uint64_t>(p.nt) * 128u >> 4);
           mma_f16_ss(dj, aj, b_desc, idesc, it != 0 ? 1u : 0u);
@@ -473,7 +483,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) lin_bf16_kernel(const __grid_c
     }
     if constexpr (kGroup == 0)
       if (e.y != nullptr && split == 0)
-        for (int j2 = 0; j2 < kMT; ++j2) linear_tile_routes(e, m0 + j2 * p.nt, min(p.nt, p.M - m0 - j2 * p.nt), tile_n, warp - 2, lane);
+        for (int j2 = 0; j2 < kMT; ++j2) linear_tile_routes(e, m0 + j2 * p.nt, min(p.nt, m_end - m0 - j2 * p.nt), tile_n, warp - 2, lane);
     bool ok = mbar_wait(bar_acc, 0, p.err, kErrWaitAcc);
     if (!ok) abort_s = 1u;
     named_bar_sync(1, 256);
@@ -565,7 +575,8 @@ __global__ void __launch_bounds__(256) lin_f32_kernel(const __grid_constant__ Li
   pdl_wait();
   __shared__ float as[16][68], ws[16][68];
   const int N = p.N_pad, K = p.K, n0 = blockIdx.x * 64;
-  int m0 = blockIdx.y * 64, m_end = p.M;
+  int m0 = blockIdx.y * 64, m_end = p.group_tiles == nullptr ? live_rows(p) : p.M;
+  if (m0 >= m_end && p.group_tiles == nullptr) return;
   const float* w = static_cast<const float*>(p.w);
   const float* a = static_cast<const float*>(p.a2 != nullptr && n0 >= p.a2_tile0 * 256 ? p.a2 : p.a);
   if (p.group_tiles != nullptr) {
@@ -612,6 +623,7 @@ __global__ void __launch_bounds__(256) lin_epi_kernel(const __grid_constant__ Li
   pdl_wait();
   const LinEpi& e = p.e;
   const int m = blockIdx.x;
+  if (p.group_tiles == nullptr && m >= live_rows(p)) return;
   const float* acc = p.ws + static_cast<size_t>(m) * p.N_pad;
   int token = m;
   if (p.group_tiles != nullptr) {                   // padding between the experts' rows: rows of no token

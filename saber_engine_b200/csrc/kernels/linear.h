@@ -78,6 +78,7 @@ struct LinParams {
   uint64_t group_w_stride;
   int group_max;        // tiles the table can hold
   LinEpi e;
+  const int32_t* live;  // rows of the step (device; 0 or null: all M).  Tiles behind them leave at once, rows behind them are not written
 };
 
 // Rows of the stream from token ids: x = table[id] * scale, an optional second copy as the operand `x0`

@@ -144,6 +144,8 @@ class StackModel:
             tiles, kb = lin.N_pad // 256 * ((M + p.nt - 1) // p.nt), lin.K // 64
             p.splits = F.stream_splits(tiles, kb)
             p.mtiles = 2 if (M > 128 and tiles > F.device_sms() and p.M_pad % 256 == 0) else 1
+        if M > 128:                                      # a bucket's padding (the head's rows are its own)
+            p.live = prog.live if lin is not self.w.head else None
         p.e = e
         prog.linear(p, tag=tag)
 
@@ -203,6 +205,7 @@ class StackModel:
         at = lambda off: blob.data_ptr() + 4 * off      # noqa: E731
         f32 = lambda *s: torch.zeros(*s, dtype=torch.float32, device=dev)   # noqa: E731
         prog = N.Program(f"{kind}-b{nseq}-w{width}")
+        prog.live = None if decode else at(lay.cu_rows + nseq)      # rows of the step
 
         # ---- activation buffers
         x = f32(M, L.round_up(W, 32))

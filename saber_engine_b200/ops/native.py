@@ -188,7 +188,7 @@ class LinEpi(C.Structure):
 class LinParams(C.Structure):
     _fields_ = [("w", P), ("a", P), ("a2", P), ("ws", P), ("counters", P), ("err", P), ("M", I), ("M_pad", I), ("N_pad", I), ("K", I), ("nt", I),
                 ("splits", I), ("fp32", I), ("fuse", I), ("mtiles", I), ("a2_tile0", I), ("group_tiles", P), ("group_ntiles", P), ("group_rows", P), ("src_row", P),
-                ("group_w_stride", U64), ("group_max", I), ("e", LinEpi)]
+                ("group_w_stride", U64), ("group_max", I), ("e", LinEpi), ("live", P)]
 
 
 class StreamEmbedParams(C.Structure):
